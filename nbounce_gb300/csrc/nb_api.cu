@@ -675,19 +675,11 @@ static int render_samples(nb_pathtracer* pt, const nb_scene* scene, const nb_cam
       if (rc) return rc;
     }
     cudaError_t e = timed_launch(pt, kKindRaygen, st, [&] { return launch_raygen(pb, wt, pt->sms, st); });
-    for (uint32_t b = 0; b <= B && e == cudaSuccess; ++b) {
-      e = timed_launch(pt, kKindTrace, st, [&] {
-        return launch_trace_wave(pb, wt, true, b, pt->d_rays, pt->sms, st, pt->d_trace_counts);
-      });
-      if (e == cudaSuccess)
-        e = timed_launch(pt, kKindShade, st, [&] {
-          if (pt->cache) return launch_shade_cache(pb, wt, cw, b, pt->sms, st);
-          if (nee) return launch_shade_nee(pb, wt, pt->sq, b, pt->sms, st);
-          return launch_shade(pb, wt, b, pt->sms, st);
-        });
-      if (e == cudaSuccess && nee)
-        e = timed_launch(pt, kKindTrace, st, [&] { return launch_trace_shadow(pb, wt, pt->sq, b, pt->sms, st); });
-    }
+    if (e == cudaSuccess)
+      e = launch_bounces(pb, wt, pt->cache ? Estimator::kCache : nee ? Estimator::kNee : Estimator::kPlain, true, B,
+                         pt->sq, cw, pt->d_rays, pt->sms, st, true, pt->d_trace_counts, [&](bool trace, auto launch) {
+                           return timed_launch(pt, trace ? kKindTrace : kKindShade, st, launch);
+                         });
     if (e == cudaSuccess && pt->cache) {
       rc = NB_OK;
       e = timed_launch(pt, kKindCacheInfer, st, [&] {

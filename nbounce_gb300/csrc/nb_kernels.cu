@@ -15,6 +15,8 @@
 //               choice, VNDF / cosine sampling, Russian roulette (pathtracing.wgsl:161-241);
 //               each block appends its survivors to the next bounce's queue grouped by
 //               direction bin (one atomic per block)
+//   paths       queues too short to fill the GPU: 8 lanes per path run it to its end, traversal and
+//               shading, in one launch (nb_group.cuh)
 //   accumulate  running mean over the batch's samples in sample order (pathtracing.wgsl:258)
 // so traversal runs in a lean kernel and the path state lives in HBM.  A wave can hold paths
 // of several jobs (render requests): tables of segments, jobs and scenes ride in the kernel
@@ -68,6 +70,27 @@ struct Hit {
   float t, u, v;
   uint32_t tri, inst;
 };
+
+// Moller-Trumbore (raytracing_sw.wgsl:51-78) on a GpuTri record (a = v0, b = e1, c = e2): calls
+// hit(t, u, v) if the ray meets the triangle closer than t_max.
+template <class OnHit>
+__device__ __forceinline__ void triangle_test(V3 ro, V3 rd, float4 a, float4 b, float4 c, float t_max, OnHit hit) {
+  const V3 e1 = xyz(b), e2 = xyz(c);
+  const V3 hv = cross(rd, e2);
+  const float det = dot(e1, hv);
+  if (det < kEps) return;
+  // det >= kEps here; 1 / det correctly rounded, as the reference arithmetic divides
+  const float inv_det = det < kRcpNewtonMax ? rcp_newton(det) : 1.0f / det;
+  const V3 sv = ro - xyz(a);
+  const float u = inv_det * dot(sv, hv);
+  if (u < 0.0f || u > 1.0f) return;
+  const V3 q = cross(sv, e1);
+  const float v = inv_det * dot(rd, q);
+  if (v < 0.0f || u + v > 1.0f) return;
+  const float t = inv_det * dot(e2, q);
+  if (t < kBias) return;
+  if (t < t_max) hit(t, u, v);
+}
 
 // Traversal state of one ray: the world ray, the current ray (world, or instance-local inside
 // a BLAS), the distance of the closest hit so far and the depth of the stack both levels share.
@@ -382,26 +405,14 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
       if (kCount) ++cnt->tris;
       const float4* tp = s.tris + 3 * (size_t)(first + j);
       const float4 a = ld4(tp), b = ld4(tp + 1), c = ld4(tp + 2);
-      const V3 e1 = xyz(b), e2 = xyz(c);
-      const V3 hv = cross(rd, e2);
-      const float det = dot(e1, hv);
-      if (det < kEps) continue;
-      // det >= kEps here; 1 / det correctly rounded, as the reference arithmetic divides
-      const float inv_det = det < kRcpNewtonMax ? rcp_newton(det) : 1.0f / det;
-      const V3 sv = ro - xyz(a);
-      const float u = inv_det * dot(sv, hv);
-      if (u < 0.0f || u > 1.0f) continue;
-      const V3 q = cross(sv, e1);
-      const float v = inv_det * dot(rd, q);
-      if (v < 0.0f || u + v > 1.0f) continue;
-      const float t = inv_det * dot(e2, q);
-      if (t < kBias) continue;
-      if (t < h_t) {
+      bool found = false;
+      triangle_test(ro, rd, a, b, c, h_t, [&](float t, float u, float v) {
         h_t = t;
         stack[kHitSlot] = make_uint2(f2u(u), f2u(v));
         stack[kHitSlot + 1] = make_uint2(f2u(b.w), cur_inst);
-        if (kAny) return false;
-      }
+        found = true;
+      });
+      if (kAny && found) return false;
     }
   }
 
@@ -479,6 +490,12 @@ __device__ __forceinline__ uint32_t trace_refill(uint32_t* fetch, uint32_t n, Lo
   return st;
 }
 
+}  // namespace nbd
+
+#include "nb_group.cuh"
+
+namespace nbd {
+
 // ------------------------------------------------------------------------------------------
 // traversal-only query (nb_trace_rays)
 // ------------------------------------------------------------------------------------------
@@ -526,6 +543,51 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? 9 : kAny ? 8 : 7)
   if (st) atomicOr(status, st);
 }
 
+
+// First work item of this group, spread over the SMs first: with fewer items than groups, every
+// warp has as few of them as possible.
+__device__ __forceinline__ uint32_t first_group_item() {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  return (lane / kGroupLanes * (kGroupThreads / 32) + warp) * gridDim.x + blockIdx.x;
+}
+// The next one of a group that wants one: *fetch counts the items taken beyond the first of every
+// group.  All lanes of the warp call it.
+__device__ __forceinline__ void next_group_item(const Group& g, uint32_t* fetch, bool want, uint32_t& i) {
+  uint32_t r = 0;
+  if (want && g.sub == 0) r = gridDim.x * kGroupsPerBlock + atomicAdd(fetch, 1u);
+  r = g.shfl(r, 0);
+  if (want) i = r;
+}
+
+// nb_trace_rays with few rays: 8 lanes per ray (GroupTrace).
+template <bool kAny>
+__global__ void __launch_bounds__(kGroupThreads, 6)
+    k_trace_rays_group(DevScene s, const float4* __restrict__ rays, uint32_t n, float4* __restrict__ hits,
+                       uint32_t* __restrict__ inst, uint32_t* __restrict__ fetch, uint32_t* __restrict__ status) {
+  __shared__ uint2 stacks[kGroupsPerBlock][kStackSize];
+  const Group g;
+  GroupTrace t;
+  uint32_t i = first_group_item();
+  bool fresh = true;
+  while (__any_sync(kWarp, i < n)) {
+    if (fresh && i < n) {
+      const float4 o = __ldg(rays + 2 * (size_t)i), d = __ldg(rays + 2 * (size_t)i + 1);
+      t.begin(s, xyz(o), xyz(d), kAny);
+      fresh = false;
+    }
+    t.step(s, g, stacks[threadIdx.x / kGroupLanes]);
+    const bool done = i < n && !t.active;
+    if (__any_sync(kWarp, done)) {
+      if (done && g.sub == 0) {
+        hits[i] = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.tri));
+        if (inst) inst[i] = t.h.inst;
+      }
+      next_group_item(g, fetch, done, i);
+      fresh = fresh || done;
+    }
+  }
+  if (t.status && g.sub == 0) atomicOr(status, t.status);
+}
 
 // ------------------------------------------------------------------------------------------
 // wavefront path tracer
@@ -647,6 +709,14 @@ __global__ void __launch_bounds__(256) k_raygen(PathBatch pb, const WaveTables w
   }
 }
 
+// Rays that the wave's per-bounce kernels trace and shade at a bounce: none if the queue is short
+// enough for k_trace_paths, which has then run its paths to their ends.
+__device__ __forceinline__ uint32_t queue_count(const PathBatch& pb, const WaveTables& wt, uint32_t bounce) {
+  if (bounce == 0) return wt.n_paths;
+  const uint32_t n = pb.counts[bounce];
+  return n <= wt.group_limit ? 0u : n;
+}
+
 // kSingle: every ray of the wave uses wt.scenes[0]; else the scene index carried in q_d.w.
 // Bounce 0 (camera rays): persistent warps take 32 consecutive queue entries per atomic - 32
 // samples of one pixel - make each lane's camera ray (camera_ray), write it to the queue for
@@ -672,12 +742,13 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? 9 : 7) k_trace_wave(P
                                                                      uint32_t bounce,
                                                        unsigned long long* __restrict__ ray_total,
                                                        unsigned long long* __restrict__ counters) {
+  const uint32_t n = queue_count(pb, wt, bounce);
+  if (n == 0) return;
   __shared__ DevScene scenes[kSingle ? 1 : nb::kMaxWaveScenes];
   if (!kSingle) {
     for (uint32_t i = threadIdx.x; i < wt.n_scenes; i += blockDim.x) scenes[i] = wt.scenes[i];
     __syncthreads();
   }
-  const uint32_t n = pb.counts[bounce];
   const float4* __restrict__ qo = (bounce & 1) ? pb.q_o[1] : pb.q_o[0];
   const float4* __restrict__ qd = (bounce & 1) ? pb.q_d[1] : pb.q_d[0];
   const int lane = threadIdx.x & 31;
@@ -1154,12 +1225,61 @@ __device__ __forceinline__ float rr_continue(uint32_t bounce, const JobParams& j
   return bounce < jp.rr_start ? 1.0f : p_continue;
 }
 
+// The ray a path continues with: origin (.w path id), direction (.w scene index), throughput
+// (.w, with environment NEE: density of the lobe sample that made the ray).
+struct NextRay {
+  float4 o, d, t;
+};
+
+// One vertex of the reference estimator (pathtracing.wgsl:161-241): radiance where the path ends
+// (end(id, L), called at most once), else the next ray; returns whether the path goes on.
+// inst() gives the hit's instance.
+template <class InstOf, class End>
+__device__ __forceinline__ bool shade_plain(const PathBatch& pb, const WaveTables& wt, const Segment* segs,
+                                            uint32_t bounce, float4 O, float4 D, float4 H, float4 Tq, InstOf inst,
+                                            End end, NextRay& next) {
+  const uint32_t id = __float_as_uint(O.w);
+  const Segment sg = segs[find_segment<false>(segs, wt.n_segs, id)];
+  const JobParams& jp = wt.jobs[sg.job];
+  const DevScene& s = wt.scenes[jp.scene];
+  V3 T = xyz(Tq);
+  const V3 rdir = xyz(D);
+  if (H.x == kNoHit) {
+    end(id, T * env_lookup(jp.env, rdir));
+    return false;
+  }
+  HitSurface hs;
+  load_hit_surface(s, inst(), O, H, rdir, hs);
+  if (hs.emissive) {  // pathtracing.wgsl:172-174
+    end(id, T * hs.color);
+    return false;
+  }
+  const uint32_t local = id - sg.path_begin;
+  const uint32_t pix = local % jp.npix;
+  const uint32_t sample = sg.first_sample + local / jp.npix;
+  float4 s0, s1;
+  bounce_samples(pb, sample, bounce, hash4f(pix % jp.width, pix / jp.width), s0, s1);
+  const BsdfSample bs = sample_bsdf<false>(hs, rdir, s0, s1);
+  T = T * bs.weight;
+  const float p_continue = rr_continue(bounce, jp, T);
+  if (s0.z < p_continue && bounce < jp.bounces) {
+    T = T / p_continue;
+    next.o = make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w);
+    next.d = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
+    next.t = make_float4(T.x, T.y, T.z, 0.0f);
+    return true;
+  }
+  end(id, V3{0.0f, 0.0f, 0.0f});  // ends without radiance
+  return false;
+}
+
 __global__ void __launch_bounds__(kShadeThreads, kShadeBlocksPerSM) k_shade(PathBatch pb, const WaveTables wt, uint32_t bounce) {
   __shared__ Segment segs[nb::kMaxWaveSegments];
   __shared__ uint32_t append_sh[2 * kDirBins];
+  const uint32_t n = queue_count(pb, wt, bounce);
+  if (n == 0) return;
   stage_segments(segs, wt);
   append_init(append_sh);
-  const uint32_t n = pb.counts[bounce];
   const bool odd = (bounce & 1) != 0;
   const float4* __restrict__ in_o = odd ? pb.q_o[1] : pb.q_o[0];
   const float4* __restrict__ in_d = odd ? pb.q_d[1] : pb.q_d[0];
@@ -1172,51 +1292,20 @@ __global__ void __launch_bounds__(kShadeThreads, kShadeBlocksPerSM) k_shade(Path
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
     const uint32_t i = base + threadIdx.x;
     bool cont = false;
-    float4 next_o = make_float4(0.f, 0.f, 0.f, 0.f), next_d = next_o, next_t = next_o;
+    NextRay next;
+    next.o = next.d = next.t = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < n) {
       const float4 O = in_o[i], D = in_d[i], H = pb.hits[i];
       const float4 Tq = bounce == 0 ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : in_t[i];
-      const uint32_t id = __float_as_uint(O.w);
-      const Segment sg = segs[find_segment<false>(segs, wt.n_segs, id)];
-      const JobParams& jp = wt.jobs[sg.job];
-      const DevScene& s = wt.scenes[jp.scene];
-      V3 T = xyz(Tq);
-      const V3 rdir = xyz(D);
-      if (H.x == kNoHit) {
-        const V3 L = T * env_lookup(jp.env, rdir);
-        pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f);
-      } else {
-        HitSurface hs;
-        load_hit_surface(s, pb.hit_inst[i], O, H, rdir, hs);
-        if (hs.emissive) {  // pathtracing.wgsl:172-174
-          const V3 L = T * hs.color;
-          pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f);
-        } else {
-          const uint32_t local = id - sg.path_begin;
-          const uint32_t pix = local % jp.npix;
-          const uint32_t sample = sg.first_sample + local / jp.npix;
-          float4 s0, s1;
-          bounce_samples(pb, sample, bounce, hash4f(pix % jp.width, pix / jp.width), s0, s1);
-          const BsdfSample bs = sample_bsdf<false>(hs, rdir, s0, s1);
-          T = T * bs.weight;
-          const float p_continue = rr_continue(bounce, jp, T);
-          if (s0.z < p_continue && bounce < jp.bounces) {
-            T = T / p_continue;
-            cont = true;
-            next_o = make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w);
-            next_d = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
-            next_t = make_float4(T.x, T.y, T.z, 0.0f);
-          } else {
-            pb.radiance[id] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // ends without radiance
-          }
-        }
-      }
+      cont = shade_plain(
+          pb, wt, segs, bounce, O, D, H, Tq, [&] { return pb.hit_inst[i]; },
+          [&](uint32_t id, V3 L) { pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f); }, next);
     }
-    const uint32_t slot = block_append_binned(pb.counts + bounce + 1, cont, next_d, append_sh);
+    const uint32_t slot = block_append_binned(pb.counts + bounce + 1, cont, next.d, append_sh);
     if (cont) {
-      out_o[slot] = next_o;
-      out_d[slot] = next_d;
-      out_t[slot] = next_t;
+      out_o[slot] = next.o;
+      out_d[slot] = next.d;
+      out_t[slot] = next.t;
     }
   }
 }
@@ -1255,14 +1344,146 @@ __device__ __forceinline__ nb::CacheFeatures cache_features(const HitSurface& hs
 //    throughput is multiplied by), continues past its query vertex for `extra` vertices and
 //    ends in a tail query that closes its radiance chain with the cache (self-training),
 //    unless a miss, an emitter or Russian roulette ends it first.
-__global__ void __launch_bounds__(kShadeExtThreads) k_shade_cache(PathBatch pb, const WaveTables wt, const nb::CacheWave cw,
+// What a vertex of the cache mode leaves behind besides radiance and the next ray: lookups and the
+// path's cache state for the next vertex (q_x of CacheWave).
+struct CacheVertex {
+  nb::CacheFeatures f;
+  V3 T;               // throughput of the image query
+  float4 x;           // next state
+  uint32_t slot;      // training slot, ~0u: none
+  bool image_q, tail_q;
+};
+
+// One vertex of the cache mode.  X: the path's state (unused at bounce 0); end(id, L) takes the
+// radiance of a path that ends without a lookup; lead: this thread writes the vertex' records
+// (the threads of a group shade the same vertex).  Returns whether the path goes on.
+template <class InstOf, class End>
+__device__ __forceinline__ bool shade_cache(const PathBatch& pb, const WaveTables& wt, const Segment* segs,
+                                            const nb::CacheWave& cw, uint32_t bounce, float4 O, float4 D, float4 H,
+                                            float4 Tq, float4 X, InstOf inst, End end, bool lead, NextRay& next,
+                                            CacheVertex& cv) {
+  const uint32_t id = __float_as_uint(O.w);
+  const Segment sg = segs[find_segment<false>(segs, wt.n_segs, id)];
+  const JobParams& jp = wt.jobs[sg.job];
+  const DevScene& s = wt.scenes[jp.scene];
+  V3 T = xyz(Tq);
+  const V3 rdir = xyz(D);
+  float budget = 0.0f, pdf_prev = 0.0f;
+  uint32_t flags = 0;
+  uint32_t& slot = cv.slot;
+  if (bounce == 0) {
+    const uint32_t G = *cw.stride;
+    const uint32_t frame_key = mix32(cw.frame ^ 0x5bd1e995u);
+    const uint32_t group = id / G;
+    const bool train = group < cw.max_slots && id % G == mix32(group ^ frame_key) % G;
+    slot = train ? group : ~0u;
+    flags = train ? nb::kPathTraining : 0u;
+  } else {
+    budget = X.x;
+    pdf_prev = X.y;
+    slot = __float_as_uint(X.z);
+    flags = __float_as_uint(X.w);
+  }
+  const bool training = (flags & nb::kPathTraining) != 0;
+  const bool image_done = (flags & nb::kPathImageDone) != 0;
+  if (H.x == kNoHit) {
+    const V3 E = env_lookup(jp.env, rdir);
+    if (!image_done) end(id, T * E);
+    if (training && lead) cw.tail[slot] = make_float4(E.x, E.y, E.z, 0.0f);
+    return false;
+  }
+  HitSurface hs;
+  load_hit_surface(s, inst(), O, H, rdir, hs);
+  if (hs.emissive) {
+    if (!image_done) end(id, T * hs.color);
+    if (training && lead) cw.tail[slot] = make_float4(hs.color.x, hs.color.y, hs.color.z, 0.0f);
+    return false;
+  }
+  const uint32_t local = id - sg.path_begin;
+  const uint32_t pix = local % jp.npix;
+  const uint32_t sample = sg.first_sample + local / jp.npix;
+  float4 s0, s1;
+  bounce_samples(pb, sample, bounce, hash4f(pix % jp.width, pix / jp.width), s0, s1);
+  const BsdfSample bs = sample_bsdf<true>(hs, rdir, s0, s1);
+  const float dist2 = H.x * H.x * dot(rdir, rdir);
+  const float cos_v = fabsf(bs.cos_o);
+  if (bounce == 0)
+    budget = cw.spread_c < 0.0f ? -1.0f : sqrtf(cw.spread_c * dist2 / (4.0f * kPi * cos_v));
+  else
+    budget = budget - sqrtf(dist2 / (pdf_prev * cos_v));
+  cv.f = cache_features(hs, bs, id);
+  cv.T = T;
+  const V3 Tn = T * bs.weight;
+  const float p_continue = rr_continue(bounce, jp, Tn);
+  const bool rr_ok = s0.z < p_continue && bounce < jp.bounces;
+  // an infinite c turns the spread rule off; otherwise NaN budgets (degenerate
+  // geometry) end the prefix as well
+  const bool spread_end = !isinf(cw.spread_c) && !(budget >= 0.0f);
+  cv.image_q = !image_done && (spread_end || bounce >= jp.bounces);
+  bool go = false;
+  if (!training) {
+    go = !cv.image_q && rr_ok;
+  } else {
+    uint32_t since = (flags >> nb::kPathSinceShift) & 0xFFu;
+    // a training path that reaches the vertex cap ends here, its pixel sample included
+    if (bounce >= nb::kCacheMaxVertices) cv.image_q = !image_done;
+    if (cv.image_q) {
+      flags |= nb::kPathImageDone;
+      since = 0;
+    }
+    if (((flags & nb::kPathImageDone) && since >= cw.extra) || bounce >= nb::kCacheMaxVertices) {
+      cv.tail_q = true;
+    } else {
+      const V3 w = rr_ok ? bs.weight / p_continue : V3{0.0f, 0.0f, 0.0f};
+      if (lead) {
+        nb::TrainVertex tv;
+        tv.f = cv.f;
+        tv.w = make_float4(w.x, w.y, w.z, 0.0f);
+        cw.verts[(size_t)slot * nb::kCacheMaxVertices + bounce] = tv;
+        cw.vert_count[slot] = bounce + 1;
+      }
+      go = rr_ok;
+      if (!go && lead) cw.tail[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (go && (flags & nb::kPathImageDone)) since += 1;
+    }
+    flags = (flags & 0xFFu) | (since << nb::kPathSinceShift);
+  }
+  if (go) {
+    const V3 Tc = Tn / p_continue;
+    next.o = make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w);
+    next.d = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
+    next.t = make_float4(Tc.x, Tc.y, Tc.z, 0.0f);
+    cv.x = make_float4(budget, bs.pdf, __uint_as_float(slot), __uint_as_float(flags));
+  }
+  return go;
+}
+
+// Writes lookup `at` of the wave (dropped beyond the capacity, which a wave's paths and training
+// slots never exceed): the pixel's query, or the tail that closes a training path's chain.
+__device__ __forceinline__ void put_image_query(const nb::CacheWave& cw, uint32_t at, const CacheVertex& cv) {
+  if (at >= cw.max_queries) return;
+  nb::CacheQuery q;
+  q.f = cv.f;
+  q.T = make_float4(cv.T.x, cv.T.y, cv.T.z, 0.0f);
+  cw.queries[at] = q;
+}
+__device__ __forceinline__ void put_tail_query(const nb::CacheWave& cw, uint32_t at, const CacheVertex& cv) {
+  if (at >= cw.max_queries) return;
+  nb::CacheQuery q;
+  q.f = cv.f;
+  q.f.tag = nb::kCacheTailBit | cv.slot;
+  q.T = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+  cw.queries[at] = q;
+}
+
+__global__ void __launch_bounds__(kShadeExtThreads, 3) k_shade_cache(PathBatch pb, const WaveTables wt, const nb::CacheWave cw,
                                                      uint32_t bounce) {
-  using nb::CacheQuery;
   __shared__ Segment segs[nb::kMaxWaveSegments];
   __shared__ uint32_t append_sh[2 * kDirBins];
+  const uint32_t n = queue_count(pb, wt, bounce);
+  if (n == 0) return;
   stage_segments(segs, wt);
   append_init(append_sh);
-  const uint32_t n = pb.counts[bounce];
   const bool odd = (bounce & 1) != 0;
   const float4* __restrict__ in_o = odd ? pb.q_o[1] : pb.q_o[0];
   const float4* __restrict__ in_d = odd ? pb.q_d[1] : pb.q_d[0];
@@ -1272,138 +1493,33 @@ __global__ void __launch_bounds__(kShadeExtThreads) k_shade_cache(PathBatch pb, 
   float4* __restrict__ out_d = odd ? pb.q_d[0] : pb.q_d[1];
   float4* __restrict__ out_t = odd ? pb.q_t[0] : pb.q_t[1];
   float4* __restrict__ out_x = odd ? cw.q_x[0] : cw.q_x[1];
-  const uint32_t G = *cw.stride;
-  const uint32_t frame_key = mix32(cw.frame ^ 0x5bd1e995u);
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
     const uint32_t i = base + threadIdx.x;
-    bool cont = false, image_q = false, tail_q = false;
-    float4 next_o = make_float4(0.f, 0.f, 0.f, 0.f), next_d = next_o, next_t = next_o, next_x = next_o;
-    nb::CacheFeatures f{};
-    V3 Tq3{0.0f, 0.0f, 0.0f};
-    uint32_t slot = ~0u;
+    bool cont = false;
+    NextRay next;
+    next.o = next.d = next.t = make_float4(0.f, 0.f, 0.f, 0.f);
+    CacheVertex cv;
+    cv.image_q = cv.tail_q = false;
     if (i < n) {
       const float4 O = in_o[i], D = in_d[i], H = pb.hits[i];
       const float4 Tq = bounce == 0 ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : in_t[i];
-      const uint32_t id = __float_as_uint(O.w);
-      const Segment sg = segs[find_segment<false>(segs, wt.n_segs, id)];
-      const JobParams& jp = wt.jobs[sg.job];
-      const DevScene& s = wt.scenes[jp.scene];
-      V3 T = xyz(Tq);
-      const V3 rdir = xyz(D);
-      float budget = 0.0f, pdf_prev = 0.0f;
-      uint32_t flags = 0;
-      if (bounce == 0) {
-        const uint32_t group = id / G;
-        const bool train = group < cw.max_slots && id % G == mix32(group ^ frame_key) % G;
-        slot = train ? group : ~0u;
-        flags = train ? nb::kPathTraining : 0u;
-      } else {
-        const float4 X = in_x[i];
-        budget = X.x;
-        pdf_prev = X.y;
-        slot = __float_as_uint(X.z);
-        flags = __float_as_uint(X.w);
-      }
-      const bool training = (flags & nb::kPathTraining) != 0;
-      const bool image_done = (flags & nb::kPathImageDone) != 0;
-      if (H.x == kNoHit) {
-        const V3 E = env_lookup(jp.env, rdir);
-        if (!image_done) {
-          const V3 L = T * E;
-          pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f);
-        }
-        if (training) cw.tail[slot] = make_float4(E.x, E.y, E.z, 0.0f);
-      } else {
-        HitSurface hs;
-        load_hit_surface(s, pb.hit_inst[i], O, H, rdir, hs);
-        if (hs.emissive) {
-          if (!image_done) {
-            const V3 L = T * hs.color;
-            pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f);
-          }
-          if (training) cw.tail[slot] = make_float4(hs.color.x, hs.color.y, hs.color.z, 0.0f);
-        } else {
-          const uint32_t local = id - sg.path_begin;
-          const uint32_t pix = local % jp.npix;
-          const uint32_t sample = sg.first_sample + local / jp.npix;
-          float4 s0, s1;
-          bounce_samples(pb, sample, bounce, hash4f(pix % jp.width, pix / jp.width), s0, s1);
-          const BsdfSample bs = sample_bsdf<true>(hs, rdir, s0, s1);
-          const float dist2 = H.x * H.x * dot(rdir, rdir);
-          const float cos_v = fabsf(bs.cos_o);
-          if (bounce == 0)
-            budget = cw.spread_c < 0.0f ? -1.0f : sqrtf(cw.spread_c * dist2 / (4.0f * kPi * cos_v));
-          else
-            budget = budget - sqrtf(dist2 / (pdf_prev * cos_v));
-          f = cache_features(hs, bs, id);
-          Tq3 = T;
-          const V3 Tn = T * bs.weight;
-          const float p_continue = rr_continue(bounce, jp, Tn);
-          const bool rr_ok = s0.z < p_continue && bounce < jp.bounces;
-          // an infinite c turns the spread rule off; otherwise NaN budgets (degenerate
-          // geometry) end the prefix as well
-          const bool spread_end = !isinf(cw.spread_c) && !(budget >= 0.0f);
-          image_q = !image_done && (spread_end || bounce >= jp.bounces);
-          bool go = false;
-          if (!training) {
-            go = !image_q && rr_ok;
-          } else {
-            uint32_t since = (flags >> nb::kPathSinceShift) & 0xFFu;
-            // a training path that reaches the vertex cap ends here, its pixel sample included
-            if (bounce >= nb::kCacheMaxVertices) image_q = !image_done;
-            if (image_q) {
-              flags |= nb::kPathImageDone;
-              since = 0;
-            }
-            if (((flags & nb::kPathImageDone) && since >= cw.extra) || bounce >= nb::kCacheMaxVertices) {
-              tail_q = true;
-            } else {
-              const V3 w = rr_ok ? bs.weight / p_continue : V3{0.0f, 0.0f, 0.0f};
-              nb::TrainVertex tv;
-              tv.f = f;
-              tv.w = make_float4(w.x, w.y, w.z, 0.0f);
-              cw.verts[(size_t)slot * nb::kCacheMaxVertices + bounce] = tv;
-              cw.vert_count[slot] = bounce + 1;
-              go = rr_ok;
-              if (!go) cw.tail[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-              if (go && (flags & nb::kPathImageDone)) since += 1;
-            }
-            flags = (flags & 0xFFu) | (since << nb::kPathSinceShift);
-          }
-          if (go) {
-            const V3 Tc = Tn / p_continue;
-            cont = true;
-            next_o = make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w);
-            next_d = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
-            next_t = make_float4(Tc.x, Tc.y, Tc.z, 0.0f);
-            next_x = make_float4(budget, bs.pdf, __uint_as_float(slot), __uint_as_float(flags));
-          }
-        }
-      }
+      const float4 X = bounce == 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : in_x[i];
+      cont = shade_cache(
+          pb, wt, segs, cw, bounce, O, D, H, Tq, X, [&] { return pb.hit_inst[i]; },
+          [&](uint32_t id, V3 L) { pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f); }, true, next, cv);
     }
-    const uint32_t at = block_append_binned(pb.counts + bounce + 1, cont, next_d, append_sh);
+    const uint32_t at = block_append_binned(pb.counts + bounce + 1, cont, next.d, append_sh);
     if (cont) {
-      out_o[at] = next_o;
-      out_d[at] = next_d;
-      out_t[at] = next_t;
-      out_x[at] = next_x;
+      out_o[at] = next.o;
+      out_d[at] = next.d;
+      out_t[at] = next.t;
+      out_x[at] = cv.x;
     }
-    const uint32_t qi = warp_append(cw.n_queries, image_q);
-    if (image_q && qi < cw.max_queries) {
-      CacheQuery q;
-      q.f = f;
-      q.T = make_float4(Tq3.x, Tq3.y, Tq3.z, 0.0f);
-      cw.queries[qi] = q;
-    }
-    const uint32_t ti = warp_append(cw.n_queries, tail_q);
-    if (tail_q && ti < cw.max_queries) {
-      CacheQuery q;
-      q.f = f;
-      q.f.tag = nb::kCacheTailBit | slot;
-      q.T = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-      cw.queries[ti] = q;
-    }
+    const uint32_t qi = warp_append(cw.n_queries, cv.image_q);
+    if (cv.image_q) put_image_query(cw, qi, cv);
+    const uint32_t ti = warp_append(cw.n_queries, cv.tail_q);
+    if (cv.tail_q) put_tail_query(cw, ti, cv);
   }
 }
 
@@ -1465,13 +1581,81 @@ __device__ __forceinline__ bool finite3(V3 v) { return isfinite(v.x) && isfinite
 // next-event estimation cannot reach a direction (below the shading normal, cos_o <= 0, a
 // mirror lobe) the carried density is +inf and the lobe sample keeps full weight, so the
 // estimator stays unbiased.  Radiance accumulates per path (+=) instead of being written once.
+//
+// One vertex: add(id, L) takes the radiance a path gains, shadow(o, d, c) the shadow ray and the
+// radiance it carries.  Returns whether the path goes on.
+template <class InstOf, class Add, class Shadow>
+__device__ __forceinline__ bool shade_nee(const PathBatch& pb, const WaveTables& wt, const Segment* segs,
+                                          uint32_t bounce, float4 O, float4 D, float4 H, float4 Tq, InstOf inst,
+                                          Add add, Shadow shadow, NextRay& next) {
+  const float kInf = __int_as_float(0x7f800000);
+  const uint32_t id = __float_as_uint(O.w);
+  const Segment sg = segs[find_segment<false>(segs, wt.n_segs, id)];
+  const JobParams& jp = wt.jobs[sg.job];
+  const DevScene& s = wt.scenes[jp.scene];
+  V3 T = xyz(Tq);
+  const V3 rdir = xyz(D);
+  if (H.x == kNoHit) {
+    V3 L = T * env_lookup(jp.env, rdir);
+    const float q = Tq.w;  // density of the lobe sample that made this ray (bounce > 0)
+    if (bounce > 0 && q < kInf) {
+      const float pe = env_pdf(jp.env, normalize(rdir));
+      L = L * (q * q / (q * q + pe * pe));
+    }
+    add(id, L);
+    return false;
+  }
+  HitSurface hs;
+  load_hit_surface(s, inst(), O, H, rdir, hs);
+  if (hs.emissive) {
+    add(id, T * hs.color);
+    return false;
+  }
+  const uint32_t local = id - sg.path_begin;
+  const uint32_t pix = local % jp.npix;
+  const uint32_t sample = sg.first_sample + local / jp.npix;
+  const float4 shift = hash4f(pix % jp.width, pix / jp.width);
+  float4 s0, s1;
+  bounce_samples(pb, sample, bounce, shift, s0, s1);
+  const BsdfSample bs = sample_bsdf<true>(hs, rdir, s0, s1);
+  // jobs without the flag take the plain estimator's exact path (one contribution
+  // added onto zero, lobe samples at full weight)
+  const bool nee_ok = (jp.flags & nb::kJobEnvNee) && bs.cos_o > 0.0f;
+  if (nee_ok) {
+    const uint32_t sb = sample * kLdsStride + 1u + bounce * kLdsPerBounce;
+    const float u1 = fract(sobol_read(pb.sobol, pb.sobol_entries, sb).w + shift.w);
+    const float u2 = fract(sobol_read(pb.sobol, pb.sobol_entries, sb + 1u).x + shift.x);
+    const V3 we = env_sample_dir(jp.env, u1, u2);
+    const float pe = env_pdf(jp.env, we);
+    if (pe > 0.0f && dot(we, bs.n) > 0.0f) {
+      const BsdfEval ev = eval_bsdf(hs, bs, we);
+      const float pe2 = pe * pe;
+      const float ws = pe2 / (ev.q_spec * ev.q_spec + pe2), wd = pe2 / (ev.q_diff * ev.q_diff + pe2);
+      const V3 C = T * env_lookup(jp.env, we) * (ev.spec * ws + ev.diff * wd) / pe;
+      if (finite3(C) && (C.x > 0.0f || C.y > 0.0f || C.z > 0.0f))
+        shadow(make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w), make_float4(we.x, we.y, we.z, D.w),
+               make_float4(C.x, C.y, C.z, 0.0f));
+    }
+  }
+  T = T * bs.weight;
+  const float p_continue = rr_continue(bounce, jp, T);
+  if (!(s0.z < p_continue && bounce < jp.bounces)) return false;
+  T = T / p_continue;
+  const float q = (nee_ok && dot(bs.wi, bs.n) > 0.0f) ? bs.pdf : kInf;
+  next.o = make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w);
+  next.d = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
+  next.t = make_float4(T.x, T.y, T.z, q);
+  return true;
+}
+
 __global__ void __launch_bounds__(kShadeExtThreads) k_shade_nee(PathBatch pb, const WaveTables wt, const ShadowQueue sq,
                                                    uint32_t bounce) {
   __shared__ Segment segs[nb::kMaxWaveSegments];
   __shared__ uint32_t append_sh[2 * kDirBins];
+  const uint32_t n = queue_count(pb, wt, bounce);
+  if (n == 0) return;
   stage_segments(segs, wt);
   append_init(append_sh);
-  const uint32_t n = pb.counts[bounce];
   const bool odd = (bounce & 1) != 0;
   const float4* __restrict__ in_o = odd ? pb.q_o[1] : pb.q_o[0];
   const float4* __restrict__ in_d = odd ? pb.q_d[1] : pb.q_d[0];
@@ -1480,85 +1664,34 @@ __global__ void __launch_bounds__(kShadeExtThreads) k_shade_nee(PathBatch pb, co
   float4* __restrict__ out_d = odd ? pb.q_d[0] : pb.q_d[1];
   float4* __restrict__ out_t = odd ? pb.q_t[0] : pb.q_t[1];
   const uint32_t stride = gridDim.x * blockDim.x;
-  const float kInf = __int_as_float(0x7f800000);
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
     const uint32_t i = base + threadIdx.x;
     bool cont = false, shadow = false;
-    float4 next_o = make_float4(0.f, 0.f, 0.f, 0.f), next_d = next_o, next_t = next_o;
-    float4 sh_o = next_o, sh_d = next_o, sh_c = next_o;
+    NextRay next;
+    next.o = next.d = next.t = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 sh_o = next.o, sh_d = next.o, sh_c = next.o;
     if (i < n) {
       const float4 O = in_o[i], D = in_d[i], H = pb.hits[i];
       const float4 Tq = bounce == 0 ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : in_t[i];
-      const uint32_t id = __float_as_uint(O.w);
-      const Segment sg = segs[find_segment<false>(segs, wt.n_segs, id)];
-      const JobParams& jp = wt.jobs[sg.job];
-      const DevScene& s = wt.scenes[jp.scene];
-      V3 T = xyz(Tq);
-      const V3 rdir = xyz(D);
-      if (H.x == kNoHit) {
-        V3 L = T * env_lookup(jp.env, rdir);
-        const float q = Tq.w;  // density of the lobe sample that made this ray (bounce > 0)
-        if (bounce > 0 && q < kInf) {
-          const float pe = env_pdf(jp.env, normalize(rdir));
-          L = L * (q * q / (q * q + pe * pe));
-        }
-        const float4 c = pb.radiance[id];
-        pb.radiance[id] = make_float4(c.x + L.x, c.y + L.y, c.z + L.z, 0.0f);
-      } else {
-        HitSurface hs;
-        load_hit_surface(s, pb.hit_inst[i], O, H, rdir, hs);
-        if (hs.emissive) {
-          const V3 L = T * hs.color;
-          const float4 c = pb.radiance[id];
-          pb.radiance[id] = make_float4(c.x + L.x, c.y + L.y, c.z + L.z, 0.0f);
-        } else {
-          const uint32_t local = id - sg.path_begin;
-          const uint32_t pix = local % jp.npix;
-          const uint32_t sample = sg.first_sample + local / jp.npix;
-          const float4 shift = hash4f(pix % jp.width, pix / jp.width);
-          float4 s0, s1;
-          bounce_samples(pb, sample, bounce, shift, s0, s1);
-          const BsdfSample bs = sample_bsdf<true>(hs, rdir, s0, s1);
-          // jobs without the flag take the plain estimator's exact path (one contribution
-          // added onto zero, lobe samples at full weight)
-          const bool nee_ok = (jp.flags & nb::kJobEnvNee) && bs.cos_o > 0.0f;
-          if (nee_ok) {
-            const uint32_t sb = sample * kLdsStride + 1u + bounce * kLdsPerBounce;
-            const float u1 = fract(sobol_read(pb.sobol, pb.sobol_entries, sb).w + shift.w);
-            const float u2 = fract(sobol_read(pb.sobol, pb.sobol_entries, sb + 1u).x + shift.x);
-            const V3 we = env_sample_dir(jp.env, u1, u2);
-            const float pe = env_pdf(jp.env, we);
-            if (pe > 0.0f && dot(we, bs.n) > 0.0f) {
-              const BsdfEval ev = eval_bsdf(hs, bs, we);
-              const float pe2 = pe * pe;
-              const float ws = pe2 / (ev.q_spec * ev.q_spec + pe2), wd = pe2 / (ev.q_diff * ev.q_diff + pe2);
-              const V3 C = T * env_lookup(jp.env, we) * (ev.spec * ws + ev.diff * wd) / pe;
-              if (finite3(C) && (C.x > 0.0f || C.y > 0.0f || C.z > 0.0f)) {
-                shadow = true;
-                sh_o = make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w);
-                sh_d = make_float4(we.x, we.y, we.z, D.w);
-                sh_c = make_float4(C.x, C.y, C.z, 0.0f);
-              }
-            }
-          }
-          T = T * bs.weight;
-          const float p_continue = rr_continue(bounce, jp, T);
-          if (s0.z < p_continue && bounce < jp.bounces) {
-            T = T / p_continue;
-            cont = true;
-            const float q = (nee_ok && dot(bs.wi, bs.n) > 0.0f) ? bs.pdf : kInf;
-            next_o = make_float4(hs.pos.x, hs.pos.y, hs.pos.z, O.w);
-            next_d = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
-            next_t = make_float4(T.x, T.y, T.z, q);
-          }
-        }
-      }
+      cont = shade_nee(
+          pb, wt, segs, bounce, O, D, H, Tq, [&] { return pb.hit_inst[i]; },
+          [&](uint32_t id, V3 L) {
+            const float4 c = pb.radiance[id];
+            pb.radiance[id] = make_float4(c.x + L.x, c.y + L.y, c.z + L.z, 0.0f);
+          },
+          [&](float4 o, float4 d, float4 c) {
+            shadow = true;
+            sh_o = o;
+            sh_d = d;
+            sh_c = c;
+          },
+          next);
     }
-    const uint32_t slot = block_append_binned(pb.counts + bounce + 1, cont, next_d, append_sh);
+    const uint32_t slot = block_append_binned(pb.counts + bounce + 1, cont, next.d, append_sh);
     if (cont) {
-      out_o[slot] = next_o;
-      out_d[slot] = next_d;
-      out_t[slot] = next_t;
+      out_o[slot] = next.o;
+      out_d[slot] = next.d;
+      out_t[slot] = next.t;
     }
     const uint32_t ss = warp_append(sq.counts + bounce, shadow);
     if (shadow) {
@@ -1576,11 +1709,12 @@ __global__ void __launch_bounds__(kShadeExtThreads) k_shade_nee(PathBatch pb, co
 // of its scene in the wave.
 __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_shadow(PathBatch pb, const WaveTables wt, const ShadowQueue sq,
                                                       uint32_t bounce) {
+  const uint32_t n = sq.counts[bounce];
+  if (n == 0) return;
   __shared__ DevScene scenes[nb::kMaxWaveScenes];
   for (uint32_t i = threadIdx.x; i < wt.n_scenes; i += blockDim.x) scenes[i] = wt.scenes[i];
   __syncthreads();
   __shared__ float world[kTraceWarps][kWorldFloats];
-  const uint32_t n = sq.counts[bounce];
   const uint32_t st = trace_refill<true, false>(
       sq.fetch + bounce, n,
       [&](uint32_t r, V3& o, V3& d, uint32_t& sidx) {
@@ -1599,6 +1733,125 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_shadow(PathBatch pb,
       },
       nullptr, world[threadIdx.x >> 5]);
   if (st) atomicOr(pb.status, st);
+}
+
+// Paths run to their ends, 8 lanes per path (GroupTrace): the camera paths of a small wave
+// (bounce0 = 0), or the queue of a bounce that no longer fills the GPU (queue_count).  Traversal and
+// shading of a path follow one another here without a launch between them, so the time is that of
+// the longest path and not the sum over the bounces of each bounce's longest ray.  All lanes of a
+// group shade the same vertex; lane 0 writes.  Samples, arithmetic and the order of a path's
+// radiance additions are those of the per-bounce kernels.  Bound by the latency of a path's steps
+// (0.8 us each) and, from ~16K paths on, by instruction issue (54%).
+enum EstimatorKind : int { kEstPlain, kEstNee, kEstCache };
+template <int kEst>
+__global__ void __launch_bounds__(kGroupThreads, 4)
+    k_trace_paths(PathBatch pb, const WaveTables wt, const nb::CacheWave cw, uint32_t bounce0,
+                  unsigned long long* __restrict__ ray_total) {
+  const uint32_t n = bounce0 == 0 ? wt.n_paths : pb.counts[bounce0];
+  if (n == 0 || (bounce0 != 0 && n > wt.group_limit)) return;
+  __shared__ Segment segs[nb::kMaxWaveSegments];
+  __shared__ uint2 stacks[kGroupsPerBlock][kStackSize];
+  stage_segments(segs, wt);
+  const Group g;
+  uint2* stack = stacks[threadIdx.x / kGroupLanes];
+  const bool lead = g.sub == 0;
+  const bool odd = (bounce0 & 1) != 0;
+  uint32_t rays = 0, b = bounce0, scene = 0;
+  GroupTrace t;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  NextRay ray;              // the ray traced (kEstNee, during a shadow ray: the one traced after it)
+  float4 X = zero;          // kEstCache: the path's state
+  float4 acc = zero;        // kEstNee: the path's radiance so far
+  V3 shadow_c{0.0f, 0.0f, 0.0f};
+  bool more = false;        // kEstNee, during a shadow ray: the path goes on after it
+  bool fresh = true;
+  uint32_t i = first_group_item();
+  while (__any_sync(kWarp, i < n)) {
+    if (fresh && i < n) {
+      if (bounce0 == 0) {
+        camera_ray(segs, wt, pb, i, ray.o, ray.d);
+        ray.t = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+        acc = zero;
+      } else {
+        ray.o = (odd ? pb.q_o[1] : pb.q_o[0])[i];
+        ray.d = (odd ? pb.q_d[1] : pb.q_d[0])[i];
+        ray.t = (odd ? pb.q_t[1] : pb.q_t[0])[i];
+        if (kEst == kEstCache) X = (odd ? cw.q_x[1] : cw.q_x[0])[i];
+        if (kEst == kEstNee) acc = pb.radiance[__float_as_uint(ray.o.w)];
+      }
+      scene = __float_as_uint(ray.d.w);
+      b = bounce0;
+      ++rays;
+      t.begin(wt.scenes[scene], xyz(ray.o), xyz(ray.d), false);
+      fresh = false;
+    }
+    t.step(wt.scenes[scene], g, stack);
+    const bool done = i < n && !t.active;
+    if (!__any_sync(kWarp, done)) continue;
+    bool ended = false;
+    if (done) {
+      bool cont;
+      if (kEst == kEstNee && t.any) {  // a shadow ray
+        if (t.h.t == kNoHit) acc = make_float4(acc.x + shadow_c.x, acc.y + shadow_c.y, acc.z + shadow_c.z, 0.0f);
+        cont = more;
+      } else {
+        const float4 H = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.tri));
+        const float4 O = ray.o, D = ray.d, T = ray.t;
+        const auto inst = [&] { return t.h.inst; };
+        const auto end = [&](uint32_t id, V3 L) {
+          if (lead) pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f);
+        };
+        if (kEst == kEstPlain) {
+          cont = shade_plain(pb, wt, segs, b, O, D, H, T, inst, end, ray);
+        } else if (kEst == kEstNee) {
+          bool shadow = false;
+          V3 so{0.0f, 0.0f, 0.0f}, sd = so;
+          cont = shade_nee(
+              pb, wt, segs, b, O, D, H, T, inst,
+              [&](uint32_t, V3 L) { acc = make_float4(acc.x + L.x, acc.y + L.y, acc.z + L.z, 0.0f); },
+              [&](float4 o, float4 d, float4 c) {
+                shadow = true;
+                so = xyz(o);
+                sd = xyz(d);
+                shadow_c = xyz(c);
+              },
+              ray);
+          if (shadow) {
+            more = cont;
+            t.begin(wt.scenes[scene], so, sd, true);
+            // a ray that traces nothing (no TLAS, non-finite) is finished at once, unoccluded
+            if (t.active) {
+              b += 1;
+              goto traced;
+            }
+            acc = make_float4(acc.x + shadow_c.x, acc.y + shadow_c.y, acc.z + shadow_c.z, 0.0f);
+          }
+        } else {
+          CacheVertex cv;
+          cv.image_q = cv.tail_q = false;
+          cont = shade_cache(pb, wt, segs, cw, b, O, D, H, T, X, inst, end, lead, ray, cv);
+          X = cv.x;
+          if (lead && cv.image_q) put_image_query(cw, atomicAdd(cw.n_queries, 1u), cv);
+          if (lead && cv.tail_q) put_tail_query(cw, atomicAdd(cw.n_queries, 1u), cv);
+        }
+        b += 1;
+      }
+      if (cont) {
+        ++rays;
+        t.begin(wt.scenes[scene], xyz(ray.o), xyz(ray.d), false);
+      } else {
+        if (kEst == kEstNee && lead) pb.radiance[__float_as_uint(ray.o.w)] = acc;
+        ended = true;
+      }
+    traced:;
+    }
+    next_group_item(g, pb.fetch + bounce0, ended, i);
+    fresh = ended;
+  }
+  if (lead) {
+    if (t.status) atomicOr(pb.status, t.status);
+    if (rays) atomicAdd(ray_total, (unsigned long long)rays);
+  }
 }
 
 __global__ void k_env_sample(const DevEnv env, const float* __restrict__ u, uint32_t n, float4* __restrict__ out) {
@@ -1649,6 +1902,15 @@ cudaError_t launch_trace_rays(const nbd::DevScene& s, const float* rays, uint32_
   cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
+  if (n <= kGroupPaths) {
+    const void* kernel = any ? (const void*)nbd::k_trace_rays_group<true> : (const void*)nbd::k_trace_rays_group<false>;
+    static const int full[2] = {blocks_for((const void*)nbd::k_trace_rays_group<false>, nbd::kGroupThreads, sms),
+                                blocks_for((const void*)nbd::k_trace_rays_group<true>, nbd::kGroupThreads, sms)};
+    const float4* r4 = (const float4*)rays;
+    float4* h4 = (float4*)hits;
+    void* args[] = {(void*)&s, (void*)&r4, (void*)&n, (void*)&h4, (void*)&inst, (void*)&fetch, (void*)&status};
+    return cudaLaunchKernel(kernel, dim3((unsigned)std::min(full[any], (int)n)), dim3(nbd::kGroupThreads), args, 0, st);
+  }
 #define NB_TRACE_RAYS(A, R)                                                                            \
   {                                                                                                    \
     static const int g = blocks_for((const void*)nbd::k_trace_rays<A, R>, nbd::kTraceThreads, sms);                  \
@@ -1717,6 +1979,21 @@ cudaError_t launch_trace_shadow(const PathBatch& pb, const WaveTables& wt, const
                                 int sms, cudaStream_t st) {
   static const int g = blocks_for((const void*)nbd::k_trace_shadow, nbd::kTraceThreads, sms);
   nbd::k_trace_shadow<<<g, nbd::kTraceThreads, 0, st>>>(pb, wt, sq, bounce);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_trace_paths(const PathBatch& pb, const WaveTables& wt, Estimator est, const CacheWave& cw,
+                               uint32_t bounce, unsigned long long* ray_total, int sms, cudaStream_t st) {
+#define NB_TRACE_PATHS(E)                                                                                  \
+  {                                                                                                        \
+    static const int g = blocks_for((const void*)nbd::k_trace_paths<E>, nbd::kGroupThreads, sms);          \
+    const int blocks = (int)std::min<uint64_t>((uint64_t)g, wt.n_paths);                                   \
+    nbd::k_trace_paths<E><<<blocks, nbd::kGroupThreads, 0, st>>>(pb, wt, cw, bounce, ray_total);           \
+  }
+  if (est == Estimator::kPlain) NB_TRACE_PATHS(nbd::kEstPlain)
+  else if (est == Estimator::kNee) NB_TRACE_PATHS(nbd::kEstNee)
+  else NB_TRACE_PATHS(nbd::kEstCache)
+#undef NB_TRACE_PATHS
   return cudaGetLastError();
 }
 

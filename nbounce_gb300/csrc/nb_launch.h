@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "nb_device.cuh"
+#include "nb_mlp.cuh"
 
 namespace nb {
 
@@ -50,7 +51,8 @@ constexpr uint32_t kTraceCounterSlots = 16;
 struct WaveTables {
   uint32_t n_segs, n_jobs, n_scenes, n_paths, n_pix;
   uint32_t flags;
-  uint32_t pad[2];
+  uint32_t group_limit;  // queues of bounces >= 1 up to this long are run to their ends by k_trace_paths
+  uint32_t pad;
   Segment segs[kMaxWaveSegments];
   JobParams jobs[kMaxWaveJobs];
   nbd::DevScene scenes[kMaxWaveScenes];
@@ -108,5 +110,56 @@ struct CacheWave;
 cudaError_t launch_shade_cache(const PathBatch& pb, const WaveTables& wt, const CacheWave& cw, uint32_t bounce,
                                int sms, cudaStream_t st);
 cudaError_t launch_accumulate(const PathBatch& pb, const WaveTables& wt, int sms, cudaStream_t st);
+
+enum class Estimator { kPlain, kNee, kCache };
+// 8 lanes per path, to its end: the camera paths of a whole wave (bounce 0), or a bounce's queue if
+// it holds at most wt.group_limit paths (the per-bounce kernels then skip that queue).
+cudaError_t launch_trace_paths(const PathBatch& pb, const WaveTables& wt, Estimator est, const CacheWave& cw,
+                               uint32_t bounce, unsigned long long* ray_total, int sms, cudaStream_t st);
+
+// Queues and waves up to this many paths, and nb_trace_rays calls up to this many rays, are traced by
+// 8 lanes per ray.  Such a ray costs ~2.5 times the instructions of a ray per lane, but a node step
+// takes 0.8 us instead of ~2, and a launch is as long as its longest ray until the GPU is full:
+// scattered rays through a 300K-triangle scene take 42 against 95 us (152 rays), 81 / 161 (9,728),
+// 165 / 193 (65,536), 286 / 238 (131,072).  With the paths run to their ends (k_trace_paths), limits
+// of 16K / 32K / 64K / 128K paths: 576x320 at 1 spp 856 / 803 / 772 / 853 us (1573 with per-bounce
+// launches alone), 256x256 at 16 spp 608 / 580 / 570 / 600 us (720), 64x48 at 1 spp 69 us (339).
+constexpr uint32_t kGroupPaths = 1u << 16;
+
+// All bounces of a wave.  groups: short queues go to k_trace_paths.  counters (optional): the
+// instrumented traversal, a ray per lane throughout.  timed(trace, launch) runs one launch (trace:
+// traversal, else shading).
+template <class Timed>
+cudaError_t launch_bounces(const PathBatch& pb, WaveTables& wt, Estimator est, bool single_scene, uint32_t max_bounces,
+                           const ShadowQueue& sq, const CacheWave& cw, unsigned long long* ray_total, int sms,
+                           cudaStream_t st, bool groups, unsigned long long* counters, Timed timed) {
+  groups = groups && counters == nullptr;
+  wt.group_limit = groups ? kGroupPaths : 0u;
+  // From bounce `last` on every queue goes to k_trace_paths, whatever its length, and the launches of
+  // later bounces are saved: there the queue holds at most kGroupPaths paths if half of the paths end
+  // per bounce (half to two thirds do in open scenes; where most survive, both ways took the same time
+  // within 10%).
+  uint32_t last = 0;
+  while (groups && (wt.n_paths >> last) > kGroupPaths) ++last;
+  cudaError_t e = cudaSuccess;
+  for (uint32_t b = 0; b <= max_bounces && e == cudaSuccess; ++b) {
+    if (groups && (b >= 1 || last == 0)) {
+      wt.group_limit = b == last ? 0xFFFFFFFFu : kGroupPaths;
+      e = timed(true, [&] { return launch_trace_paths(pb, wt, est, cw, b, ray_total, sms, st); });
+      if (b == last) return e;
+    }
+    if (e == cudaSuccess)
+      e = timed(true, [&] { return launch_trace_wave(pb, wt, single_scene, b, ray_total, sms, st, counters); });
+    if (e == cudaSuccess)
+      e = timed(false, [&] {
+        return est == Estimator::kCache ? launch_shade_cache(pb, wt, cw, b, sms, st)
+               : est == Estimator::kNee ? launch_shade_nee(pb, wt, sq, b, sms, st)
+                                        : launch_shade(pb, wt, b, sms, st);
+      });
+    if (e == cudaSuccess && est == Estimator::kNee)
+      e = timed(true, [&] { return launch_trace_shadow(pb, wt, sq, b, sms, st); });
+  }
+  return e;
+}
 
 }  // namespace nb

@@ -323,17 +323,20 @@ struct nb_server {
     return false;
   }
 
+  // A small wave stays on the per-bounce kernels: with 8 lanes per path the server drains small jobs
+  // about as fast as a caller can submit them, and a queue limit would then not shed any (a burst of
+  // 200 jobs of 64x64 pixels at 16,384 paths per wave).
+  bool group_wave() const { return wt->n_paths > 4 * kGroupPaths; }
+
   cudaError_t launch_wave(uint32_t max_bounces, bool single_scene, bool nee) {
     PathBatch p = pb;
     cudaError_t e = cudaSuccess;
     wt->flags = nee ? kWaveZeroRadiance : 0u;  // NEE shading adds to radiance
     if (nee) e = cudaMemsetAsync(sq.counts, 0, 2 * kMaxBounceSlots * sizeof(uint32_t), stream);
     if (e == cudaSuccess) e = launch_raygen(p, *wt, sms, stream);
-    for (uint32_t b = 0; b <= max_bounces && e == cudaSuccess; ++b) {
-      e = launch_trace_wave(p, *wt, single_scene, b, d_rays, sms, stream);
-      if (e == cudaSuccess) e = nee ? launch_shade_nee(p, *wt, sq, b, sms, stream) : launch_shade(p, *wt, b, sms, stream);
-      if (e == cudaSuccess && nee) e = launch_trace_shadow(p, *wt, sq, b, sms, stream);
-    }
+    if (e == cudaSuccess)
+      e = launch_bounces(p, *wt, nee ? Estimator::kNee : Estimator::kPlain, single_scene, max_bounces, sq, CacheWave{},
+                         d_rays, sms, stream, group_wave(), nullptr, [](bool, auto launch) { return launch(); });
     if (e == cudaSuccess) e = launch_accumulate(p, *wt, sms, stream);
     return e;
   }
@@ -357,10 +360,9 @@ struct nb_server {
     PathBatch p = pb;
     wt->flags = kWaveZeroRadiance;  // cache lookups add to radiance
     cudaError_t e = launch_raygen(p, *wt, sms, stream);
-    for (uint32_t b = 0; b <= max_bounces && e == cudaSuccess; ++b) {
-      e = launch_trace_wave(p, *wt, true, b, d_rays, sms, stream);
-      if (e == cudaSuccess) e = launch_shade_cache(p, *wt, cw, b, sms, stream);
-    }
+    if (e == cudaSuccess)
+      e = launch_bounces(p, *wt, Estimator::kCache, true, max_bounces, sq, cw, d_rays, sms, stream, group_wave(), nullptr,
+                         [](bool, auto launch) { return launch(); });
     if (e != cudaSuccess) return cuda_fail(e, "cache wave launch");
     if ((rc = cache_wave_infer(c, p, sms, stream)) || (rc = cache_wave_train(c, wt->n_paths, sms, stream)))
       return rc;

@@ -142,10 +142,9 @@ extern "C" int nb_render_static(const nb_scene* scene, const nb_env* env, const 
     wt.n_paths = (uint32_t)npix * S;
     wt.n_pix = (uint32_t)npix;
     e = launch_raygen(pb, wt, sms, st);
-    for (uint32_t b = 0; b <= bounces && e == cudaSuccess; ++b) {
-      e = launch_trace_wave(pb, wt, true, b, rays, sms, st);
-      if (e == cudaSuccess) e = launch_shade(pb, wt, b, sms, st);
-    }
+    if (e == cudaSuccess)
+      e = launch_bounces(pb, wt, Estimator::kPlain, true, bounces, ShadowQueue{}, CacheWave{}, rays, sms, st, true, nullptr,
+                         [](bool, auto launch) { return launch(); });
     if (e == cudaSuccess) e = launch_accumulate(pb, wt, sms, st);
     done += S;
   }
