@@ -58,9 +58,9 @@ TRACE_ISSUE_ACTIVE_PCT = {"camera_rays": 77.4, "bounce_1": 75.3}
 UNIT = "Mrays/s"
 WORKLOAD = "instanced 16 meshes / 1024 instances, 1920x1080, 64 spp, 8 bounces, equirect sky"
 # bytes the device layout fetches per unit of traversal work (nb_trace_counters): an 8-wide
-# node, a triangle record, an instance record, a stack entry written and read back; plus the
+# node, a triangle (half of a leaf slot's 80 bytes), an instance record, a stack entry written and read back; plus the
 # ray read from the queue (two float4) and the hit written (float4 + instance id)
-NODE_BYTES, TRI_BYTES, INST_BYTES, PUSH_BYTES, RAY_IO_BYTES = 80, 48, 64, 16, 52
+NODE_BYTES, TRI_BYTES, INST_BYTES, PUSH_BYTES, RAY_IO_BYTES = 80, 40, 64, 16, 52
 TRUTH_DIR = os.path.join(ROOT, "tests", "golden")
 
 
@@ -623,7 +623,7 @@ def trace_roofline(pt, scene, cam, env, desc, kt, steps, rays_per_step, sh, of):
     """Roofline of the traversal kernel from one instrumented frame outside the timed region.
 
     achieved = the bytes the device's own layout fetches per trace launch (80 B per 8-wide node
-    test, 48 B per triangle test, 64 B per instance entry, 16 B per stack entry written and read
+    test, 40 B per triangle test, 64 B per instance entry, 16 B per stack entry written and read
     back, 52 B of ray in / hit out), counted by nb_trace_counters, divided by the timed average
     trace launch duration; peak = the measured HBM copy bandwidth.  Most of those bytes are
     served by L1 and L2, so frac is the kernel's distance from the memory roofline, and the

@@ -271,7 +271,7 @@ int nb_pathtracer_enable_timing(nb_pathtracer* pt, int enable);
 int nb_pathtracer_kernel_times(nb_pathtracer* pt, nb_kernel_times* out, int reset, void* stream);
 
 /* Traversal work counters, per bounce: what the device's own layout fetches for the closest-hit
- * queries of that bounce - 80-byte 8-wide nodes (TLAS and BLAS), 48-byte triangle records,
+ * queries of that bounce - 80-byte 8-wide nodes (TLAS and BLAS), triangles (80 bytes per one or two),
  * 64-byte instance records - and the 8-byte stack entries pushed (each popped once).  While
  * enabled, renders run an instrumented copy of the traversal kernel (same results, slower);
  * the measurement counterpart of the reference's n_aabb / n_tri counters

@@ -106,7 +106,7 @@ static int upload_scene(nb_scene* s) {
   const WideNode *wb = nullptr, *wt = nullptr;
   const GpuInstTrace* it = nullptr;
   const GpuInstShade* is = nullptr;
-  const GpuTri* tr = nullptr;
+  const GpuTriPair* tr = nullptr;
   const GpuVAttr* va = nullptr;
   const uint32_t* ti = nullptr;
   if ((st = s->arena.upload(h.wblas, &wb)) || (st = s->arena.upload(h.wtlas, &wt)) ||
@@ -122,7 +122,7 @@ static int upload_scene(nb_scene* s) {
   d.vattr = (const float4*)va;
   d.tri_idx = ti;
   d.has_tlas = h.has_tlas ? 1u : 0u;
-  d.n_tris = (uint32_t)h.tris.size();
+  d.n_tris = (uint32_t)(h.indices.size() / 3);
   d.n_inst = (uint32_t)h.itrace.size();
   d.n_vertices = (uint32_t)h.vertices.size();
   void* p = nullptr;
@@ -135,7 +135,7 @@ static int upload_scene(nb_scene* s) {
   h.wtlas_nodes = h.wtlas.size();
   std::vector<WideNode>().swap(h.wblas);
   std::vector<WideNode>().swap(h.wtlas);
-  std::vector<GpuTri>().swap(h.tris);
+  std::vector<GpuTriPair>().swap(h.tris);
   std::vector<GpuVAttr>().swap(h.vattr);
   s->sms = sm_count();
   return NB_OK;

@@ -133,11 +133,11 @@ __device__ __forceinline__ float nb_acos(float y) { return nb_atan2(sqrtf((1.0f 
 
 // Device view of a scene (pointers into library-owned device memory).
 struct DevScene {
-  const float4* tlas_wide;    // 5 float4 per 8-wide TLAS node; the root is node 0
-  const float4* blas_wide;    // 5 float4 per 8-wide BLAS node
+  const float4* tlas_wide;    // 6 float4 per 8-wide TLAS node; the root is node 0
+  const float4* blas_wide;    // 6 float4 per 8-wide BLAS node
   const float4* inst_trace;   // 4 float4 per instance, in wide-TLAS leaf order
   const float4* inst_shade;   // 6 float4 per instance, reference (TLAS-permuted) order
-  const float4* tris;         // 3 float4 per triangle, in wide-BLAS leaf order
+  const float4* tris;         // 6 float4 per leaf slot (GpuTriPair), in wide-BLAS leaf order
   const uint32_t* tri_idx;    // 3 vertex ids per reference triangle
   const float4* vattr;        // 2 float4 per vertex
   uint32_t has_tlas;

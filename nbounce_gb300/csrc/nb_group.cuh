@@ -114,7 +114,8 @@ struct GroupTrace {
       if (__any_sync(kWarp, enter)) {
         if (enter) {  // transform the world ray (raytracing_sw.wgsl:202-206)
           const float4* it = s.inst_trace + 4 * (size_t)(node & ~kInstanceBit);
-          const float4 r0 = ld4(it), r1 = ld4(it + 1), r2 = ld4(it + 2), r3 = ld4(it + 3);
+          const F8 i0 = ld8(it), i1 = ld8(it + 2);
+          const float4 r0 = i0.a, r1 = i0.b, r2 = i1.a, r3 = i1.b;
           ro = V3{r0.x * wo.x + r0.y * wo.y + r0.z * wo.z + r0.w * 1.0f,
                   r1.x * wo.x + r1.y * wo.y + r1.z * wo.z + r1.w * 1.0f,
                   r2.x * wo.x + r2.y * wo.y + r2.z * wo.z + r2.w * 1.0f};
@@ -135,14 +136,13 @@ struct GroupTrace {
     // the near plane is the low one where the direction is positive
     float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     uint2 base = make_uint2(0u, 0u);
-    uint32_t meta = 0, nx = 0, ny = 0, nz = 0, fx = 0, fy = 0, fz = 0;
+    uint32_t nx = 0, ny = 0, nz = 0, fx = 0, fy = 0, fz = 0;
     if (active) {
-      const unsigned char* p = (const unsigned char*)((in_blas ? s.blas_wide : s.tlas_wide) + 5 * (size_t)node);
+      const unsigned char* p = (const unsigned char*)((in_blas ? s.blas_wide : s.tlas_wide) + 6 * (size_t)node);
       const uint32_t x = rinv.x >= 0.0f ? 0u : 24u, y = rinv.y >= 0.0f ? 0u : 24u, z = rinv.z >= 0.0f ? 0u : 24u;
       q0 = __ldg((const float4*)p);
       base = __ldg((const uint2*)(p + 16));
       p += g.sub;
-      meta = __ldg(p + 24);
       nx = __ldg(p + 32 + x);
       ny = __ldg(p + 40 + y);
       nz = __ldg(p + 48 + z);
@@ -165,11 +165,13 @@ struct GroupTrace {
                            fmaf(plane_float(fz), az, cz + dz));
     const float lo = fmaxf(tn, 0.0f);
     const float t_below = __uint_as_float(f2u(h.t) - 1u);
-    const bool hit = meta != 0u && lo <= fminf(tf, t_below);
-    const bool inner = (meta & 0x80u) != 0u;
+    const uint32_t n_inner = eb >> 28;
+    const bool hit = g.sub < ((eb >> 24) & 15u) && lo <= fminf(tf, t_below);
+    const bool inner = g.sub < n_inner;
     const bool leaf = hit && in_blas && !inner, push = hit && !leaf;
     const uint32_t key = push ? (f2u(lo) & ~7u) | g.sub : 0xFFFFFFFFu;
-    const uint32_t ref = inner ? base.x + (meta & 7u) : (kInstanceBit | (base.y + (meta & 31u)));
+    const uint32_t slot = base.y + g.sub - n_inner;  // of a leaf child
+    const uint32_t ref = inner ? base.x + g.sub : kInstanceBit | slot;
 
     // ---- rank the hit children; the nearest inner child is visited next, the others pushed ----
     const uint32_t pm = g.ballot(push);
@@ -199,19 +201,14 @@ struct GroupTrace {
       uint32_t btri = 0;
       bool better = false;
       if (leaf) {
-        const uint32_t prim = base.y + (meta & 31u), n_prim = meta >> 5;
-        for (uint32_t j = 0; j < n_prim; ++j) {
-          const float4* tp = s.tris + 3 * (size_t)(prim + j);
-          const float4 a = ld4(tp), b = ld4(tp + 1), c = ld4(tp + 2);
-          triangle_test(ro, rd, a, b, c, bt, [&](float t, float u, float v) {
-            bt = t;
-            bu = u;
-            bv = v;
-            btri = f2u(b.w);
-            better = true;
-          });
-          if (any && better) break;
-        }
+        triangle_pair_test(ro, rd, s.tris + 6 * (size_t)slot, bt, [&](float t, float u, float v, uint32_t tri) {
+          if (any && better) return;  // any hit: the first
+          bt = t;
+          bu = u;
+          bv = v;
+          btri = tri;
+          better = true;
+        });
       }
       const uint32_t bm = g.ballot(better);
       if (__any_sync(kWarp, bm != 0u)) {

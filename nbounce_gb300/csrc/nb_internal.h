@@ -5,14 +5,14 @@
 // vertices and a u32 index list, and its traversal loads both children of an inner node as
 // two separate 32-byte nodes and every triangle through three indexed 48-byte vertex loads
 // (raytracing_sw.wgsl:218-225, 275-279).  The device layout keeps the same trees but packs
-// what one traversal step touches into 16-byte-aligned records read with 128-bit loads:
-//   WideNode     80 B  8 children of a collapsed node: 8-bit quantised boxes, slot metadata
-//   GpuTri       48 B  v0, e1 = v1 - v0, e2 = v2 - v0 (the subtractions intersect_triangle
-//                      performs) + the reference triangle index
+// what one traversal step touches into 32-byte-aligned records read with 256-bit loads:
+//   WideNode     96 B  8 children of a collapsed node: 8-bit quantised boxes
+//   GpuTriPair   96 B  the one or two triangles of a leaf slot: v0, e1 = v1 - v0, e2 = v2 - v0 (the
+//                      subtractions intersect_triangle performs) + the reference triangle indices
 //   GpuInstTrace 64 B  the three rows of world_to_local used to transform rays, BLAS root,
 //                      reference instance index
 //   GpuInstShade 96 B  what intersect_scene/shading read from an instance
-//   GpuVAttr     32 B  vertex normal + tangent (positions live in GpuTri)
+//   GpuVAttr     32 B  vertex normal + tangent (positions live in GpuTriPair)
 // Triangles and instances are stored in the order of the wide trees' leaves.
 #pragma once
 
@@ -29,15 +29,14 @@ constexpr uint32_t kLdsStride = 17u;      // pathtracing.wgsl:4 (fixed, independ
 constexpr uint32_t kLdsPerBounce = 2u;    // pathtracing.wgsl:2
 constexpr uint32_t kMaxSampleCount = 1024u;  // pathtracer.rs:56
 
-struct alignas(16) GpuTri {
-  float v0[3];
-  uint32_t pad0;
-  float e1[3];
-  uint32_t ref_index;  // index in the reference's permuted triangle list (reported by hits)
-  float e2[3];
-  uint32_t pad2;
+// The triangles of a leaf slot, one or two, component by component: [0] and [1] are the lanes of the
+// packed triangle test.  A slot of one triangle has a degenerate second one (all zero: det = 0).
+struct alignas(32) GpuTriPair {
+  float v0[3][2], e1[3][2], e2[3][2];
+  uint32_t ref_index[2];  // index in the reference's permuted triangle list (reported by hits)
+  uint32_t pad[4];
 };
-struct alignas(16) GpuInstTrace {
+struct alignas(32) GpuInstTrace {
   float row[3][4];     // row r = (W[0][r], W[1][r], W[2][r], W[3][r]) of world_to_local
   uint32_t blas_root;  // root of the instance's BLAS in the wide BLAS node array
   uint32_t ref_index;  // TLAS-permuted instance index of the reference (reported by hits)
@@ -53,23 +52,27 @@ struct alignas(16) GpuVAttr {
   float t[3];
   float pad;
 };
-// 8-wide node collapsed from the reference's binary tree (80 B = 5 x 16 B).  Child boxes are
+// 8-wide node collapsed from the reference's binary tree (96 B).  Child boxes are
 // quantised to 8 bits per plane on a per-axis power-of-two grid anchored at p; the quantised
-// boxes contain the exact ones.  meta[k]: 0 = empty slot; 0x80 | r = inner child at
-// child_base + r; (n << 5) | o = leaf of n (1..3) primitives at prim_base + o.
-struct alignas(16) WideNode {
+// boxes contain the exact ones.  The inner children come first: slot k is the inner child at
+// child_base + k for k < n_inner, and up to n_children the leaf slot at prim_base + k - n_inner (a
+// GpuTriPair in a BLAS, a GpuInstTrace in the TLAS).
+struct alignas(32) WideNode {
   float p[3];
   uint8_t e[3];        // biased exponent of the grid step per axis (float bits e << 23)
-  uint8_t n_children;
+  uint8_t counts;      // n_children | n_inner << 4
   uint32_t child_base;
   uint32_t prim_base;
-  uint8_t meta[8];
+  uint32_t pad[2];
   uint8_t qlo_x[8], qlo_y[8], qlo_z[8], qhi_x[8], qhi_y[8], qhi_z[8];
+  uint32_t pad2[4];
+  uint32_t n_children() const { return counts & 15u; }
+  uint32_t n_inner() const { return counts >> 4; }
 };
-static_assert(sizeof(WideNode) == 80, "WideNode");
+static_assert(sizeof(WideNode) == 96, "WideNode");
 constexpr uint32_t kInstanceBit = 0x80000000u;  // TLAS stack entry that names an instance
 
-static_assert(sizeof(GpuTri) == 48, "GpuTri");
+static_assert(sizeof(GpuTriPair) == 96, "GpuTriPair");
 static_assert(sizeof(GpuInstTrace) == 64, "GpuInstTrace");
 static_assert(sizeof(GpuInstShade) == 96, "GpuInstShade");
 static_assert(sizeof(GpuVAttr) == 32, "GpuVAttr");
@@ -89,7 +92,7 @@ struct HostScene {
   bool has_tlas = false;
   std::vector<GpuInstTrace> itrace;
   std::vector<GpuInstShade> ishade;
-  std::vector<GpuTri> tris;
+  std::vector<GpuTriPair> tris;
   std::vector<GpuVAttr> vattr;
   double build_ms = 0.0;
 };

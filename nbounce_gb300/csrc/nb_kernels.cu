@@ -8,7 +8,7 @@
 //   trace       persistent warps take 32 rays at a time with one atomic and walk 8-wide
 //               quantised trees (raytracing_sw.wgsl:176-319): BLASes collapsed from the
 //               reference's, a TLAS over tight world boxes of the instances (large instances
-//               split at their BLAS root).  One 80-byte node load tests eight child boxes; hit
+//               split at their BLAS root).  One node load (80 bytes) tests eight child boxes; hit
 //               children are pushed in distance order so the nearest is visited next, then the
 //               node's hit leaf triangles are tested
 //   shade       hit attributes (raytracing_sw.wgsl:138-173), env/emission termination, lobe
@@ -52,6 +52,17 @@ constexpr uint32_t kInstanceBit = 0x80000000u;
 
 __device__ __forceinline__ float4 ld4(const float4* p) { return __ldg(p); }
 __device__ __forceinline__ uint32_t f2u(float x) { return __float_as_uint(x); }
+// A 32-byte sector in one load (32-byte aligned).
+struct F8 {
+  float4 a, b;
+};
+__device__ __forceinline__ F8 ld8(const float4* p) {
+  F8 v;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v.a.x), "=f"(v.a.y), "=f"(v.a.z), "=f"(v.a.w), "=f"(v.b.x), "=f"(v.b.y), "=f"(v.b.z), "=f"(v.b.w)
+      : "l"(p));
+  return v;
+}
 
 // Direction reciprocal for box tests only: components below 1e-20 in magnitude are nudged to
 // +-1e-20 so that every plane distance stays finite (triangle tests use the true direction).
@@ -71,25 +82,92 @@ struct Hit {
   uint32_t tri, inst;
 };
 
-// Moller-Trumbore (raytracing_sw.wgsl:51-78) on a GpuTri record (a = v0, b = e1, c = e2): calls
-// hit(t, u, v) if the ray meets the triangle closer than t_max.
+// Two floats in a register pair and arithmetic on both: one instruction for two IEEE operations,
+// each rounded as the scalar one.
+struct F2 {
+  uint64_t r;
+};
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+  F2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v.r) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ F2 pack2(uint32_t lo, uint32_t hi) {
+  F2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v.r) : "r"(lo), "r"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(F2 v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v.r));
+  return f;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v.r) : "l"(a.r), "l"(b.r), "l"(c.r));
+  return v;
+}
+// The product is taken as fma(a, b, -0), the same value and sign: a packed multiplication that meets
+// a packed addition is contracted into one FMA even with -fmad=false (and so is one whose -0 the
+// compiler can see, hence the constant bank), which would change the hit's bits.
+__constant__ float2 kNegZero2 = {-0.0f, -0.0f};
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return fma2(a, b, pack2(kNegZero2.x, kNegZero2.y)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  F2 v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v.r) : "l"(a.r), "l"(b.r));
+  return v;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+  F2 v;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v.r) : "l"(a.r), "l"(b.r));
+  return v;
+}
+struct V3x2 {
+  F2 x, y, z;
+};
+__device__ __forceinline__ V3x2 both(V3 v) { return V3x2{pack2(v.x, v.x), pack2(v.y, v.y), pack2(v.z, v.z)}; }
+__device__ __forceinline__ V3x2 operator-(V3x2 a, V3x2 b) { return V3x2{a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ F2 dot(V3x2 a, V3x2 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ V3x2 cross(V3x2 a, V3x2 b) {
+  return V3x2{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+}
+
+// Moller-Trumbore (raytracing_sw.wgsl:51-78) on the two triangles of a leaf slot at once
+// (GpuTriPair): the operations and roundings of the two tests one after the other.  Calls
+// hit(t, u, v, triangle) for the first if it is closer than t_max, then for the second if it is
+// closer than that.  The records' loads are issued together and the arithmetic is packed, so a slot
+// costs one round trip and about 90 instructions instead of two and 130.
 template <class OnHit>
-__device__ __forceinline__ void triangle_test(V3 ro, V3 rd, float4 a, float4 b, float4 c, float t_max, OnHit hit) {
-  const V3 e1 = xyz(b), e2 = xyz(c);
-  const V3 hv = cross(rd, e2);
-  const float det = dot(e1, hv);
-  if (det < kEps) return;
-  // det >= kEps here; 1 / det correctly rounded, as the reference arithmetic divides
-  const float inv_det = det < kRcpNewtonMax ? rcp_newton(det) : 1.0f / det;
-  const V3 sv = ro - xyz(a);
-  const float u = inv_det * dot(sv, hv);
-  if (u < 0.0f || u > 1.0f) return;
-  const V3 q = cross(sv, e1);
-  const float v = inv_det * dot(rd, q);
-  if (v < 0.0f || u + v > 1.0f) return;
-  const float t = inv_det * dot(e2, q);
-  if (t < kBias) return;
-  if (t < t_max) hit(t, u, v);
+__device__ __forceinline__ void triangle_pair_test(V3 ro, V3 rd, const float4* p, float t_max, OnHit hit) {
+  const F8 s0 = ld8(p), s1 = ld8(p + 2);
+  const float4 p0 = s0.a, p1 = s0.b, p2 = s1.a, p3 = s1.b, p4 = ld4(p + 4);
+  const V3x2 v0{pack2(p0.x, p0.y), pack2(p0.z, p0.w), pack2(p1.x, p1.y)};
+  const V3x2 e1{pack2(p1.z, p1.w), pack2(p2.x, p2.y), pack2(p2.z, p2.w)};
+  const V3x2 e2{pack2(p3.x, p3.y), pack2(p3.z, p3.w), pack2(p4.x, p4.y)};
+  const V3x2 d = both(rd);
+  const V3x2 hv = cross(d, e2);
+  const F2 det2 = dot(e1, hv);
+  const float2 det = unpack2(det2);
+  const bool back0 = det.x < kEps, back1 = det.y < kEps;
+  if (back0 && back1) return;
+  // a det that counts is >= kEps; 1 / det correctly rounded, as the reference arithmetic divides
+  float2 inv{rcp_newton(det.x), rcp_newton(det.y)};
+  if (!(fmaxf(det.x, det.y) < kRcpNewtonMax)) inv = make_float2(1.0f / det.x, 1.0f / det.y);
+  const F2 inv2 = pack2(inv.x, inv.y);
+  const V3x2 sv = both(ro) - v0;
+  const F2 u2 = inv2 * dot(sv, hv);
+  const V3x2 q = cross(sv, e1);
+  const F2 v2 = inv2 * dot(d, q);
+  const float2 u = unpack2(u2), v = unpack2(v2), uv = unpack2(u2 + v2);
+  const bool out0 = back0 || u.x < 0.0f || u.x > 1.0f || v.x < 0.0f || uv.x > 1.0f;
+  const bool out1 = back1 || u.y < 0.0f || u.y > 1.0f || v.y < 0.0f || uv.y > 1.0f;
+  if (out0 && out1) return;
+  const float2 t = unpack2(inv2 * dot(e2, q));
+  if (!out0 && !(t.x < kBias) && t.x < t_max) {
+    t_max = t.x;
+    hit(t.x, u.x, v.x, f2u(p4.z));
+  }
+  if (!out1 && !(t.y < kBias) && t.y < t_max) hit(t.y, u.y, v.y, f2u(p4.w));
 }
 
 // Traversal state of one ray: the world ray, the current ray (world, or instance-local inside
@@ -98,7 +176,7 @@ __device__ __forceinline__ void triangle_test(V3 ro, V3 rd, float4 a, float4 b, 
 // the rest of the hit record (u, v, triangle, instance), written only when a closer hit is
 // found, lives in two extra slots at the end of that array (kHitSlot), and the world ray's
 // reciprocal direction is recomputed when a BLAS is left - both to keep the state within the
-// register budget of 8 resident blocks of 128 threads.
+// register budget (kRefillBlocks, kChunkBlocks).
 constexpr int kHitSlot = kStackSize;  // stack[kHitSlot] = (u, v), stack[kHitSlot + 1] = (tri, inst)
 struct TraceState {
   V3 wo, wd;
@@ -146,6 +224,12 @@ __device__ __forceinline__ void trace_begin(TraceState& t, uint2* stack, const D
 constexpr int kWorldFloats = 9 * 32;
 constexpr int kTraceWarps = 4;  // every traversal kernel runs blocks of 128 threads
 constexpr int kTraceThreads = 32 * kTraceWarps;
+// Blocks per SM of the traversal kernels: with lane refill 7 (72 registers), whole-warp chunks 6 (80).
+// The packed test of a slot's two triangles needs the registers; with one block more the kernels spill
+// 40-140 bytes.  1920x1080 at 64 spp (1.2M triangles) / scattered any hit and camera rays on the
+// 1M-triangle soup, refill and chunk blocks 9+7: 118.0 / 6.06 / 2.54 ms, 8+7: 115.7 / 5.67 / 2.54,
+// 7+6: 110.4 / 5.02 / 2.53, 6+5: 114.4 / 5.05 / 2.66.
+constexpr int kRefillBlocks = 7, kChunkBlocks = 6;
 struct WorldRegs {
   const TraceState& t;
   __device__ __forceinline__ V3 o() const { return t.wo; }
@@ -189,8 +273,8 @@ struct WorldShared {
 };
 
 // Work counters of the instrumented traversal (kCount instantiations only): what the device
-// layout fetches per ray - 80-byte wide nodes of the TLAS and the BLASes, 48-byte triangle
-// records, 64-byte instance records - and the 8-byte stack entries pushed (each later popped);
+// layout fetches per ray - 80 bytes of the wide nodes of the TLAS and the BLASes, the triangles of
+// leaf slots (80 bytes for one or two), 64-byte instance records - and the 8-byte stack entries pushed (each later popped);
 // and how the lanes of a warp share the node steps: warp steps (lanes that test a node
 // together count one step, recorded by the lowest of them) with their lanes, and of those the
 // steps in which some lane tests leaf triangles, with the lanes that do and the largest
@@ -203,6 +287,16 @@ __device__ __forceinline__ bool lowest_active(uint32_t mask) {
   return (threadIdx.x & 31u) == (uint32_t)(__ffs(mask) - 1);
 }
 
+// Bound by instruction issue and the ALU pipe for camera rays (75% / 75% of peak, 22 of 32 lanes
+// active) and by latency and divergence for secondary rays (66%, 16 of 32).  What it costs per warp
+// step is its instructions, most of them not in the box tests: a slot's triangles are tested two at a
+// time (triangle_pair_test), the box tests take a child's near and far plane of an axis in one packed
+// FMA, and a hit child's stack entry is one addition (inner children come first in a node, so the slot
+// is the offset) stored at a fixed place below the batch's top.  Against one triangle at a time,
+// slot metadata and a branch per pushed child, at the same sizes as above: 1920x1080 at 64 spp 116.6 ->
+// 110.4 ms, camera rays on the soup 2.67 -> 2.53, scattered any hit 5.42 -> 5.02, closest (1M rays)
+// 1.94 -> 1.71 ms.
+//
 // One traversal step: pop the next entry when no node is pending, then test one 8-wide node
 // and its leaf triangles.  Returns false once the ray is finished (stack empty, an any-hit
 // found, or the iteration cap reached).  wr gives the world ray (WorldRegs, WorldMixed or
@@ -235,12 +329,13 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
       }
       --sp;
       const uint2 e = stack[sp];
-      if (__uint_as_float(e.y) >= h_t) continue;  // raytracing_sw.wgsl:197,271
+      if (__uint_as_float(e.y & ~7u) >= h_t) continue;  // raytracing_sw.wgsl:197,271
       if (!in_blas && (e.x & kInstanceBit)) {
         // enter an instance: transform the world ray (raytracing_sw.wgsl:202-206)
         if (kCount) ++cnt->insts;
         const float4* it = s.inst_trace + 4 * (size_t)(e.x & ~kInstanceBit);
-        const float4 r0 = ld4(it), r1 = ld4(it + 1), r2 = ld4(it + 2), r3 = ld4(it + 3);
+        const F8 i0 = ld8(it), i1 = ld8(it + 2);
+        const float4 r0 = i0.a, r1 = i0.b, r2 = i1.a, r3 = i1.b;
         const V3 wo = wr.o(), wd = wr.d();
         ro = V3{r0.x * wo.x + r0.y * wo.y + r0.z * wo.z + r0.w * 1.0f,
                 r1.x * wo.x + r1.y * wo.y + r1.z * wo.z + r1.w * 1.0f,
@@ -270,8 +365,10 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
       cnt->lane_steps += (uint32_t)__popc(together);
     }
   }
-  const float4* np = (in_blas ? s.blas_wide : s.tlas_wide) + 5 * (size_t)node;
-  const float4 q0 = ld4(np), q1 = ld4(np + 1), q2 = ld4(np + 2), q3 = ld4(np + 3), q4 = ld4(np + 4);
+  const float4* np = (in_blas ? s.blas_wide : s.tlas_wide) + 6 * (size_t)node;
+  const F8 w0 = ld8(np), w1 = ld8(np + 2);
+  const float4 q0 = w0.a, q2 = w1.a, q3 = w1.b, q4 = ld4(np + 4);
+  const uint2 q1 = make_uint2(f2u(w0.b.x), f2u(w0.b.y));
   const uint32_t eb = f2u(q0.w);
   const float ax = __uint_as_float((eb & 0xFFu) << 23) * rinv.x;
   const float ay = __uint_as_float(((eb >> 8) & 0xFFu) << 23) * rinv.y;
@@ -292,8 +389,8 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
   const float dz = fmaf(fabsf(az), 0.0078125f, fabsf(bz) * 1.9073486328125e-6f);
   const float cx = fmaf(-32768.0f, ax, bx), cy = fmaf(-32768.0f, ay, by), cz = fmaf(-32768.0f, az, bz);
   const float cnx = cx - dx, cfx = cx + dx, cny = cy - dy, cfy = cy + dy, cnz = cz - dz, cfz = cz + dz;
-  const uint32_t child_base = f2u(q1.x), prim_base = f2u(q1.y);
-  const uint32_t m0 = f2u(q1.z), m1 = f2u(q1.w);
+  const uint32_t child_base = q1.x, prim_base = q1.y;
+  const uint32_t n_inner = eb >> 28;
   // near/far planes per axis by the sign of the direction: the near plane of a child is its
   // low plane where rinv >= 0 (t grows with the quantised coordinate), else its high plane
   const bool pxs = rinv.x >= 0.0f, pys = rinv.y >= 0.0f, pzs = rinv.z >= 0.0f;
@@ -305,33 +402,33 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
   const uint32_t fz0 = pzs ? f2u(q4.z) : f2u(q3.x), fz1 = pzs ? f2u(q4.w) : f2u(q3.y);
   // a child is hit when max(tn, 0) <= min(tf, the largest float below the closest hit)
   const float t_below = __uint_as_float(f2u(h_t) - 1u);  // h_t > 0
+  // a child's near and far plane of an axis in one packed FMA
+  const F2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+  const F2 cx2 = pack2(cnx, cfx), cy2 = pack2(cny, cfy), cz2 = pack2(cnz, cfz);
   uint32_t key[8];
-  uint32_t leaf_mask = 0, n_push = 0;
+  uint32_t hits = 0;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     // byte k of the plane words as the float 2^15 + q: bits 0x4700qq00
     const uint32_t sel = 0x7404u + ((uint32_t)(k & 3) << 4);
-    const uint32_t meta = __byte_perm(k < 4 ? m0 : m1, 0u, 0x4440u + (uint32_t)(k & 3));
-    const float nx = __uint_as_float(__byte_perm(k < 4 ? nx0 : nx1, 0x47000000u, sel));
-    const float fx = __uint_as_float(__byte_perm(k < 4 ? fx0 : fx1, 0x47000000u, sel));
-    const float ny = __uint_as_float(__byte_perm(k < 4 ? ny0 : ny1, 0x47000000u, sel));
-    const float fy = __uint_as_float(__byte_perm(k < 4 ? fy0 : fy1, 0x47000000u, sel));
-    const float nz = __uint_as_float(__byte_perm(k < 4 ? nz0 : nz1, 0x47000000u, sel));
-    const float fz = __uint_as_float(__byte_perm(k < 4 ? fz0 : fz1, 0x47000000u, sel));
-    const float tn = fmaxf(fmaxf(fmaf(nx, ax, cnx), fmaf(ny, ay, cny)), fmaf(nz, az, cnz));
-    const float tf = fminf(fminf(fmaf(fx, ax, cfx), fmaf(fy, ay, cfy)), fmaf(fz, az, cfz));
-    const float lo = fmaxf(tn, 0.0f);
-    const bool hit = meta != 0u && lo <= fminf(tf, t_below);
-    key[k] = 0xFFFFFFFFu;
-    if (hit) {
-      if (in_blas && !(meta & 0x80u)) {
-        leaf_mask |= 1u << k;
-      } else {
-        key[k] = (f2u(lo) & ~7u) | (uint32_t)k;
-        ++n_push;
-      }
-    }
+    auto planes = [&](uint32_t n0, uint32_t n1, uint32_t f0, uint32_t f1) {
+      return pack2(__byte_perm(k < 4 ? n0 : n1, 0x47000000u, sel), __byte_perm(k < 4 ? f0 : f1, 0x47000000u, sel));
+    };
+    const float2 tx = unpack2(fma2(planes(nx0, nx1, fx0, fx1), ax2, cx2));
+    const float2 ty = unpack2(fma2(planes(ny0, ny1, fy0, fy1), ay2, cy2));
+    const float2 tz = unpack2(fma2(planes(nz0, nz1, fz0, fz1), az2, cz2));
+    const float lo = fmaxf(fmaxf(fmaxf(tx.x, ty.x), tz.x), 0.0f);
+    const float hi = fminf(fminf(fminf(tx.y, ty.y), tz.y), t_below);
+    if (lo <= hi) hits |= 1u << k;
+    key[k] = (f2u(lo) & ~7u) | (uint32_t)k;
   }
+  hits &= (1u << ((eb >> 24) & 15u)) - 1u;
+  const uint32_t inner = in_blas ? (1u << n_inner) - 1u : 0xFFu;  // children that are visited, not tested
+  uint32_t leaf_mask = hits & ~inner;
+  const uint32_t push_mask = hits & inner;
+  const int n_push = __popc(push_mask);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) key[k] = (push_mask & (1u << k)) ? key[k] : 0xFFFFFFFFu;
 
   // The hit children are ordered and pushed before the node's leaf triangles are tested:
   // the keys' registers are free again during the triangle loads (measured 1.6% faster than
@@ -344,49 +441,56 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
   key[j] = max(key[i], key[j]);                    \
   key[i] = lo_;                                    \
 }
-  // push far to near; the nearest inner child is visited next without a push
-  auto take = [&](uint32_t kk, bool nearest) {
-    const float d = __uint_as_float(kk & ~7u);
-    const uint32_t slot = kk & 7u;
-    const uint32_t meta = ((slot < 4 ? m0 : m1) >> (8 * (slot & 3))) & 0xFFu;
-    const uint32_t ref = (meta & 0x80u) ? child_base + (meta & 7u) : (kInstanceBit | (prim_base + (meta & 31u)));
-    if (nearest && (meta & 0x80u)) {
-      node = ref;
-      have_node = true;
-      next_d = d;
-    } else if (sp < kStackSize) {
-      stack[sp] = make_uint2(ref, kk & ~7u);
-      ++sp;
-      if (kCount) ++cnt->pushes;
+  if (n_push > 0) {
+    if (n_push == 1) {  // the single hit child: no sort
+#pragma unroll
+      for (int k = 1; k < 8; ++k) key[0] = min(key[0], key[k]);
     } else {
-      status |= kStatusStackOverflow;
+      NB_CX(0, 2) NB_CX(1, 3) NB_CX(4, 6) NB_CX(5, 7)
+      NB_CX(0, 4) NB_CX(1, 5) NB_CX(2, 6) NB_CX(3, 7)
+      NB_CX(0, 1) NB_CX(2, 3) NB_CX(4, 5) NB_CX(6, 7)
+      NB_CX(2, 4) NB_CX(3, 5)
+      NB_CX(1, 4) NB_CX(3, 6)
+      NB_CX(1, 2) NB_CX(3, 4) NB_CX(5, 6)
     }
-  };
-  if (n_push == 1) {  // the single hit child: no sort, no loop over the empty keys
-    uint32_t m = key[0];
+    // a child's stack entry: node or instance index and its key (its slot in the low 3 bits)
+    const uint32_t inst_base = kInstanceBit + prim_base - n_inner;
+    auto entry = [&](uint32_t kk) {
+      const uint32_t slot = kk & 7u;
+      return make_uint2((slot < n_inner ? child_base : inst_base) + slot, kk);
+    };
+    // far to near, the nearest at top; the nearest inner child is visited next without a push
+    const int top = sp + n_push - 1;
+    const uint2 first = entry(key[0]);
+    have_node = !(first.x & kInstanceBit);
+    if (top < kStackSize) {
 #pragma unroll
-    for (int k = 1; k < 8; ++k) m = min(m, key[k]);
-    take(m, true);
-  } else if (n_push > 1) {
-    NB_CX(0, 2) NB_CX(1, 3) NB_CX(4, 6) NB_CX(5, 7)
-    NB_CX(0, 4) NB_CX(1, 5) NB_CX(2, 6) NB_CX(3, 7)
-    NB_CX(0, 1) NB_CX(2, 3) NB_CX(4, 5) NB_CX(6, 7)
-    NB_CX(2, 4) NB_CX(3, 5)
-    NB_CX(1, 4) NB_CX(3, 6)
-    NB_CX(1, 2) NB_CX(3, 4) NB_CX(5, 6)
+      for (int k = 1; k < 8; ++k)
+        if (k < n_push) stack[top - k] = entry(key[k]);
+      if (!have_node) stack[top] = first;
+      sp = have_node ? top : top + 1;
+    } else {
+      // the last entries that fit (key[k] with a variable k would put the keys in memory)
 #pragma unroll
-    for (int k = 7; k >= 0; --k) {
-      if (key[k] != 0xFFFFFFFFu) take(key[k], k == 0);
+      for (int k = 7; k >= 0; --k) {
+        if (k >= n_push || (k == 0 && have_node)) continue;
+        if (sp < kStackSize) stack[sp++] = entry(key[k]);
+        else status |= kStatusStackOverflow;
+      }
+    }
+    if (kCount) cnt->pushes += (uint32_t)(n_push - (have_node ? 1 : 0));
+    if (have_node) {
+      node = first.x;
+      next_d = __uint_as_float(first.y & ~7u);
     }
   }
 #undef NB_CX
   if (kCount) {
     const uint32_t together = __activemask();
     uint32_t n_tris = 0;
-    for (uint32_t lm = leaf_mask; lm; lm &= lm - 1) {
-      const int k = __ffs(lm) - 1;
-      n_tris += (((k < 4 ? m0 : m1) >> (8 * (k & 3))) & 0xFFu) >> 5;
-    }
+    for (uint32_t lm = leaf_mask; lm; lm &= lm - 1)
+      n_tris += f2u(ld4(s.tris + 6 * (size_t)(prim_base + (uint32_t)(__ffs(lm) - 1) - n_inner) + 4).w) == 0xFFFFFFFFu ? 1u : 2u;
+    cnt->tris += n_tris;
     const uint32_t with_leaves = __ballot_sync(together, leaf_mask != 0u);
     const uint32_t most = __reduce_max_sync(together, n_tris);
     if (with_leaves && lowest_active(together)) {
@@ -397,23 +501,18 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
   }
   // ---- BLAS leaves: Moller-Trumbore (raytracing_sw.wgsl:51-78, 274-286) ----
   while (leaf_mask) {
-    const int k = __ffs(leaf_mask) - 1;
+    const uint32_t k = (uint32_t)(__ffs(leaf_mask) - 1);
     leaf_mask &= leaf_mask - 1;
-    const uint32_t meta = ((k < 4 ? m0 : m1) >> (8 * (k & 3))) & 0xFFu;
-    const uint32_t first = prim_base + (meta & 31u), n = meta >> 5;
-    for (uint32_t j = 0; j < n; ++j) {
-      if (kCount) ++cnt->tris;
-      const float4* tp = s.tris + 3 * (size_t)(first + j);
-      const float4 a = ld4(tp), b = ld4(tp + 1), c = ld4(tp + 2);
-      bool found = false;
-      triangle_test(ro, rd, a, b, c, h_t, [&](float t, float u, float v) {
-        h_t = t;
-        stack[kHitSlot] = make_uint2(f2u(u), f2u(v));
-        stack[kHitSlot + 1] = make_uint2(f2u(b.w), cur_inst);
-        found = true;
-      });
-      if (kAny && found) return false;
-    }
+    bool found = false;
+    triangle_pair_test(ro, rd, s.tris + 6 * (size_t)(prim_base + k - n_inner), h_t,
+                       [&](float t, float u, float v, uint32_t tri) {
+                         if (kAny && found) return;  // any hit: the first
+                         h_t = t;
+                         stack[kHitSlot] = make_uint2(f2u(u), f2u(v));
+                         stack[kHitSlot + 1] = make_uint2(tri, cur_inst);
+                         found = true;
+                       });
+    if (kAny && found) return false;
   }
 
   if (have_node && next_d >= h_t) have_node = false;  // a leaf above is closer than the next node
@@ -500,11 +599,9 @@ namespace nbd {
 // traversal-only query (nb_trace_rays)
 // ------------------------------------------------------------------------------------------
 // kRefill: lanes refill as they finish (trace_refill), for rays whose neighbours in the array
-// are unrelated; else each warp traces 32 consecutive rays to the end.  Blocks per SM: 9 with
-// refill (56 registers; 1M-triangle soup, incoherent rays: 28.0 -> 26.8 ms against 8 blocks),
-// 8 for any hit without refill (64 registers), 7 for closest hit without refill (72).
+// are unrelated; else each warp traces 32 consecutive rays to the end.
 template <bool kAny, bool kRefill>
-__global__ void __launch_bounds__(kTraceThreads, kRefill ? 9 : kAny ? 8 : 7)
+__global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChunkBlocks)
     k_trace_rays(DevScene s, const float4* __restrict__ rays, uint32_t n, float4* __restrict__ hits,
                  uint32_t* __restrict__ inst, uint32_t* __restrict__ fetch, uint32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
@@ -733,12 +830,9 @@ __device__ __forceinline__ uint32_t queue_count(const PathBatch& pb, const WaveT
 // differ widely, so without refill most lanes idle while the longest ray finishes (11 of 32
 // lanes active per instruction on bounce 1).  Camera rays keep whole-warp chunks: a warp's 32
 // samples of one pixel finish together, and refilling them measured 9% slower traversal.
-// Refill changes only which lane traces a ray, not its result.  The refill instantiation runs
-// 9 blocks of 128 per SM at 56 registers (8 bytes spilled); per benchmark frame 8 blocks at 64
-// registers took 1.2 ms longer and 10 at 48 (100 bytes spilled) 4.7 ms longer: secondary rays
-// wait on dependent loads, and more warps hide them.
+// Refill changes only which lane traces a ray, not its result.
 template <bool kSingle, bool kCount, bool kRefill>
-__global__ void __launch_bounds__(kTraceThreads, kRefill ? 9 : 7) k_trace_wave(PathBatch pb, const WaveTables wt,
+__global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChunkBlocks) k_trace_wave(PathBatch pb, const WaveTables wt,
                                                                      uint32_t bounce,
                                                        unsigned long long* __restrict__ ray_total,
                                                        unsigned long long* __restrict__ counters) {
@@ -1707,7 +1801,7 @@ __global__ void __launch_bounds__(kShadeExtThreads) k_shade_nee(PathBatch pb, co
 // refill (trace_refill); unoccluded rays add their contribution to the path.  A path has at most one shadow ray per bounce, so
 // each radiance entry has one writer per launch.  .w of a shadow ray's direction is the index
 // of its scene in the wave.
-__global__ void __launch_bounds__(kTraceThreads, 8) k_trace_shadow(PathBatch pb, const WaveTables wt, const ShadowQueue sq,
+__global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(PathBatch pb, const WaveTables wt, const ShadowQueue sq,
                                                       uint32_t bounce) {
   const uint32_t n = sq.counts[bounce];
   if (n == 0) return;

@@ -567,7 +567,7 @@ namespace {
 // Each reference tree is collapsed into a tree of 8-wide nodes.  Leaf slots are the maximal
 // subtrees of at most max_leaf contiguous primitives (a reference leaf with more counts as an
 // inner node over its two contiguous halves): 2 triangles in a BLAS, 1 instance in the TLAS
-// (the slot metadata holds at most 3).  Which binary nodes become wide nodes is chosen by the
+// (a GpuTriPair).  Which binary nodes become wide nodes is chosen by the
 // SAH-optimal dynamic programme of Ylitie, Karras and Laine 2017 ("Efficient incoherent ray
 // traversal on GPUs through compressed wide BVHs", section 3): C(x, i) is the least cost of
 // covering the subtree of x with at most i child slots, where a leaf slot costs nothing (every
@@ -593,13 +593,15 @@ struct Item {
   }
 };
 
+constexpr uint32_t kNoPrim = 0xFFFFFFFFu;
 struct Collapser {
   const std::vector<nb_bvh_node>& ref;
   // primitive boxes (float), indexed by reference primitive index
   const std::vector<float>& prim_box;  // 6 floats per primitive: min xyz, max xyz
   std::vector<WideNode>* out;
   std::vector<uint32_t>* prim_order;   // new order -> reference primitive index
-  uint32_t max_leaf;                   // primitives per leaf slot (2 triangles, 1 instance; <= 3)
+  uint32_t max_leaf;                   // primitives per leaf slot (2 triangles, 1 instance); each
+                                       // slot takes max_leaf entries of prim_order, ~0u: none
 
   struct Span {
     uint32_t first = 0xFFFFFFFFu, end = 0, count = 0;
@@ -793,28 +795,24 @@ struct Collapser {
       } else {
         items.push_back(cur);
       }
+      std::stable_partition(items.begin(), items.end(), [&](int32_t x) { return dp[x].l >= 0; });
       WideNode w{};
       std::vector<Item> slots;
       w.child_base = (uint32_t)out->size();
-      w.prim_base = (uint32_t)prim_order->size();
-      uint32_t n_inner = 0, offset = 0;
+      w.prim_base = (uint32_t)(prim_order->size() / max_leaf);
+      uint32_t n_inner = 0;
       for (const int32_t x : items) {
         const Item& it = dp[x].it;
-        uint8_t meta;
         if (dp[x].l >= 0) {
-          meta = (uint8_t)(0x80u | n_inner);
           ++n_inner;
           queue.push_back(x);
           out->push_back(WideNode{});
         } else {
-          meta = (uint8_t)((it.count << 5) | offset);
-          for (uint32_t i = it.start; i < it.start + it.count; ++i) prim_order->push_back(i);
-          offset += it.count;
+          for (uint32_t i = 0; i < max_leaf; ++i) prim_order->push_back(i < it.count ? it.start + i : kNoPrim);
         }
-        w.meta[slots.size()] = meta;
         slots.push_back(it);
       }
-      w.n_children = (uint8_t)slots.size();
+      w.counts = (uint8_t)(slots.size() | n_inner << 4);
       quantise(&w, slots);
       (*out)[self] = w;
     }
@@ -917,15 +915,14 @@ std::vector<TlasEntry> tlas_entries(const HostScene& s, const std::vector<uint32
   for (size_t i = 0; i < s.instances.size(); ++i) {
     const uint32_t root = s.wblas_root[inst_blas[i]];
     const WideNode& w = s.wblas[root];
-    bool split = w.n_children > 1;
-    for (int k = 0; k < w.n_children; ++k) split = split && (w.meta[k] & 0x80u);
+    bool split = w.n_children() > 1 && w.n_inner() == w.n_children();
     if (split) {
       float ib[6];
       instance_box(s.instances[i], s.blas[s.instances[i].node], ib);
       split = area(ib, ib + 3) > kRebraidArea * scene;
     }
     if (split) {
-      for (int k = 0; k < w.n_children; ++k) e.push_back({(uint32_t)i, w.child_base + (w.meta[k] & 7u)});
+      for (uint32_t k = 0; k < w.n_children(); ++k) e.push_back({(uint32_t)i, w.child_base + k});
     } else {
       e.push_back({(uint32_t)i, root});
     }
@@ -956,15 +953,15 @@ void entry_boxes(const HostScene& s, const std::vector<uint32_t>& tri_order, con
     while (!st.empty()) {
       const WideNode& w = s.wblas[st.back()];
       st.pop_back();
-      for (int c = 0; c < w.n_children; ++c) {
-        const uint32_t meta = w.meta[c];
-        if (meta & 0x80u) {
-          st.push_back(w.child_base + (meta & 7u));
+      for (uint32_t c = 0; c < w.n_children(); ++c) {
+        if (c < w.n_inner()) {
+          st.push_back(w.child_base + c);
           continue;
         }
-        const uint32_t first = w.prim_base + (meta & 31u), cnt = meta >> 5;
-        for (uint32_t j = 0; j < cnt; ++j) {
-          const uint32_t t = tri_order[first + j];
+        const size_t pair = w.prim_base + c - w.n_inner();
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t t = tri_order[2 * pair + j];
+          if (t == kNoPrim) continue;
           for (int q = 0; q < 3; ++q) {
             const uint32_t vi = s.indices[3 * (size_t)t + q];
             if (!mark[vi]) {
@@ -1076,7 +1073,7 @@ int to_device_layout(HostScene* s) {
     for (size_t k = 0; k < roots.size(); ++k) collapse(k);
   }
   for (size_t k = 0; k < roots.size(); ++k) {
-    const uint32_t node_off = (uint32_t)s->wblas.size(), prim_off = (uint32_t)tri_order.size();
+    const uint32_t node_off = (uint32_t)s->wblas.size(), prim_off = (uint32_t)(tri_order.size() / 2);
     s->wblas_root.push_back(node_off);
     for (WideNode w : wide[k]) {
       w.child_base += node_off;
@@ -1087,17 +1084,18 @@ int to_device_layout(HostScene* s) {
     std::vector<WideNode>().swap(wide[k]);
     std::vector<uint32_t>().swap(order[k]);
   }
-  s->tris.assign(tri_order.size(), GpuTri{});
-  parallel_for(tri_order.size(), [&](size_t k) {
-    const uint32_t t = tri_order[k];
-    const float* a = s->vertices[s->indices[3 * t]].position;
-    const float* b = s->vertices[s->indices[3 * t + 1]].position;
-    const float* c = s->vertices[s->indices[3 * t + 2]].position;
-    GpuTri& g = s->tris[k];
-    for (int q = 0; q < 3; ++q) { g.v0[q] = a[q]; g.e1[q] = b[q] - a[q]; g.e2[q] = c[q] - a[q]; }
-    g.pad0 = 0;
-    g.ref_index = t;
-    g.pad2 = 0;
+  s->tris.assign(tri_order.size() / 2, GpuTriPair{});
+  parallel_for(s->tris.size(), [&](size_t k) {
+    GpuTriPair& g = s->tris[k];
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t t = tri_order[2 * k + j];
+      g.ref_index[j] = t;
+      if (t == kNoPrim) continue;
+      const float* a = s->vertices[s->indices[3 * (size_t)t]].position;
+      const float* b = s->vertices[s->indices[3 * (size_t)t + 1]].position;
+      const float* c = s->vertices[s->indices[3 * (size_t)t + 2]].position;
+      for (int q = 0; q < 3; ++q) { g.v0[q][j] = a[q]; g.e1[q][j] = b[q] - a[q]; g.e2[q][j] = c[q] - a[q]; }
+    }
   });
   s->vattr.resize(nv);
   parallel_for(nv, [&](size_t i) {
