@@ -272,6 +272,37 @@ struct WorldShared {
   __device__ __forceinline__ void set_inv(V3 r) const { set_world_inv(w + 192, r); }
 };
 
+// Where a ray's stack entries lie.  LocalStack: all in thread-local memory (whole-warp chunks: a
+// warp's rays are at nearly the same depth, 92% of the loads hit L1, and a node step is then often the
+// same single hit child for all lanes, which needs no sort).  SharedStack (lane refill): the first
+// kSharedEntries in shared memory, entry-major (conflict-free at any mix of depths), deeper ones in
+// local memory.  Scattered rays' local stacks miss L1 (16% hits on the 1M-triangle soup, half on the
+// benchmark frame's bounce 1), and a pop then waits for L2 before the node's own load can start.  8 /
+// 12 / 16 / 20 entries: scattered any hit on the soup 5.15 / 4.78 / 4.60 / 4.58 ms (all local 5.02),
+// 1920x1080 at 64 spp 110.3 / 106.5 / 106.6 / 107.0 (110.4).  Without the single-child branch the
+// scattered rays take 4.51 ms (camera rays, which keep it, 2.53 instead of 2.60).
+constexpr int kSharedEntries = 16;
+struct LocalStack {
+  static constexpr bool kScattered = false;
+  static constexpr int kFast = kStackSize, kStride = 1;
+  uint2* local;
+  __device__ __forceinline__ uint2* fast(int top) const { return local + top; }
+  __device__ __forceinline__ uint2 get(int i) const { return local[i]; }
+  __device__ __forceinline__ void put(int i, uint2 e) const { local[i] = e; }
+};
+struct SharedStack {
+  static constexpr bool kScattered = true;
+  static constexpr int kFast = kSharedEntries, kStride = kTraceThreads;
+  uint2* local;
+  uint2* sh;  // this thread's column
+  __device__ __forceinline__ uint2* fast(int top) const { return sh + top * kStride; }
+  __device__ __forceinline__ uint2 get(int i) const { return i < kFast ? sh[i * kStride] : local[i]; }
+  __device__ __forceinline__ void put(int i, uint2 e) const {
+    if (i < kFast) sh[i * kStride] = e;
+    else local[i] = e;
+  }
+};
+
 // Work counters of the instrumented traversal (kCount instantiations only): what the device
 // layout fetches per ray - 80 bytes of the wide nodes of the TLAS and the BLASes, the triangles of
 // leaf slots (80 bytes for one or two), 64-byte instance records - and the 8-byte stack entries pushed (each later popped);
@@ -301,8 +332,8 @@ __device__ __forceinline__ bool lowest_active(uint32_t mask) {
 // and its leaf triangles.  Returns false once the ray is finished (stack empty, an any-hit
 // found, or the iteration cap reached).  wr gives the world ray (WorldRegs, WorldMixed or
 // WorldShared).
-template <bool kAny, bool kCount, class World>
-__device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const DevScene& s, TraceCount* cnt,
+template <bool kAny, bool kCount, class World, class Stack>
+__device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, const DevScene& s, TraceCount* cnt,
                                            const World& wr) {
   if (t.iter > kIterationCap) {
     t.status |= kStatusIterationCap;
@@ -328,7 +359,7 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
         break;
       }
       --sp;
-      const uint2 e = stack[sp];
+      const uint2 e = stack.get(sp);
       if (__uint_as_float(e.y & ~7u) >= h_t) continue;  // raytracing_sw.wgsl:197,271
       if (!in_blas && (e.x & kInstanceBit)) {
         // enter an instance: transform the world ray (raytracing_sw.wgsl:202-206)
@@ -442,7 +473,7 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
   key[i] = lo_;                                    \
 }
   if (n_push > 0) {
-    if (n_push == 1) {  // the single hit child: no sort
+    if (!Stack::kScattered && n_push == 1) {  // the single hit child: no sort
 #pragma unroll
       for (int k = 1; k < 8; ++k) key[0] = min(key[0], key[k]);
     } else {
@@ -463,18 +494,19 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
     const int top = sp + n_push - 1;
     const uint2 first = entry(key[0]);
     have_node = !(first.x & kInstanceBit);
-    if (top < kStackSize) {
+    if (top < Stack::kFast) {
+      uint2* at = stack.fast(top);
 #pragma unroll
       for (int k = 1; k < 8; ++k)
-        if (k < n_push) stack[top - k] = entry(key[k]);
-      if (!have_node) stack[top] = first;
+        if (k < n_push) at[-k * Stack::kStride] = entry(key[k]);
+      if (!have_node) at[0] = first;
       sp = have_node ? top : top + 1;
     } else {
-      // the last entries that fit (key[k] with a variable k would put the keys in memory)
+      // one by one, the last ones only as far as they fit
 #pragma unroll
       for (int k = 7; k >= 0; --k) {
         if (k >= n_push || (k == 0 && have_node)) continue;
-        if (sp < kStackSize) stack[sp++] = entry(key[k]);
+        if (sp < kStackSize) stack.put(sp++, entry(key[k]));
         else status |= kStatusStackOverflow;
       }
     }
@@ -508,8 +540,8 @@ __device__ __forceinline__ bool trace_step(TraceState& t, uint2* stack, const De
                        [&](float t, float u, float v, uint32_t tri) {
                          if (kAny && found) return;  // any hit: the first
                          h_t = t;
-                         stack[kHitSlot] = make_uint2(f2u(u), f2u(v));
-                         stack[kHitSlot + 1] = make_uint2(tri, cur_inst);
+                         stack.local[kHitSlot] = make_uint2(f2u(u), f2u(v));
+                         stack.local[kHitSlot + 1] = make_uint2(tri, cur_inst);
                          found = true;
                        });
     if (kAny && found) return false;
@@ -526,7 +558,7 @@ __device__ __forceinline__ uint32_t trace_ray(const DevScene& s, const V3 wo, co
   TraceState t;
   uint2 stack[kStackSize + 2];
   trace_begin(t, stack, s, wo, wd);
-  while (trace_step<kAny, kCount>(t, stack, s, cnt, WorldRegs{t})) {
+  while (trace_step<kAny, kCount>(t, LocalStack{stack}, s, cnt, WorldRegs{t})) {
   }
   const uint2 uv = stack[kHitSlot], ti = stack[kHitSlot + 1];
   h.t = t.t_hit;
@@ -550,7 +582,7 @@ __device__ __forceinline__ uint32_t trace_ray(const DevScene& s, const V3 wo, co
 constexpr uint32_t kRefillIdle = 6;
 template <bool kAny, bool kCount, class Load, class SceneOf, class Finish>
 __device__ __forceinline__ uint32_t trace_refill(uint32_t* fetch, uint32_t n, Load load, SceneOf scene, Finish finish,
-                                                 TraceCount* cnt, float* world) {
+                                                 TraceCount* cnt, float* world, uint2* entries) {
   const WorldShared wr{world};
   const uint32_t lane = threadIdx.x & 31u;
   TraceState t;
@@ -578,7 +610,7 @@ __device__ __forceinline__ uint32_t trace_refill(uint32_t* fetch, uint32_t n, Lo
         }
       }
     }
-    if (my != kNone && !trace_step<kAny, kCount>(t, stack, scene(sidx), cnt, wr)) {
+    if (my != kNone && !trace_step<kAny, kCount>(t, SharedStack{stack, entries}, scene(sidx), cnt, wr)) {
       finish(my, t.t_hit, stack[kHitSlot], stack[kHitSlot + 1]);
       st |= t.status;
       my = kNone;
@@ -608,6 +640,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChun
   uint32_t st = 0;
   if (kRefill) {
     __shared__ float world[kTraceWarps][kWorldFloats];
+    __shared__ uint2 entries[kSharedEntries][kTraceThreads];
     st = trace_refill<kAny, false>(
         fetch, n,
         [&](uint32_t r, V3& o, V3& d, uint32_t& sidx) {
@@ -620,7 +653,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChun
           hits[r] = make_float4(t_hit, __uint_as_float(uv.x), __uint_as_float(uv.y), __uint_as_float(ti.x));
           if (inst) inst[r] = ti.y;
         },
-        nullptr, world[threadIdx.x >> 5]);
+        nullptr, world[threadIdx.x >> 5], &entries[0][threadIdx.x]);
   } else {
     while (true) {
       uint32_t base = 0;
@@ -869,7 +902,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChun
         trace_begin(t, stack, sc0, xyz(o), xyz(d));
         set_world_inv(inv_c[threadIdx.x >> 5], t.rinv);
         const WorldMixed wm{t, inv_c[threadIdx.x >> 5]};
-        while (trace_step<false, kCount>(t, stack, sc0, &cnt, wm)) {
+        while (trace_step<false, kCount>(t, LocalStack{stack}, sc0, &cnt, wm)) {
         }
         st |= t.status;
         const uint2 uv = stack[kHitSlot], ti = stack[kHitSlot + 1];
@@ -879,6 +912,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChun
     }
   } else {
     __shared__ float world[kTraceWarps][kWorldFloats];
+    __shared__ uint2 entries[kSharedEntries][kTraceThreads];
     const DevScene* sc = kSingle ? wt.scenes : scenes;
     st = trace_refill<false, kCount>(
         pb.fetch + bounce, n,
@@ -893,7 +927,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChun
           pb.hits[r] = make_float4(t_hit, __uint_as_float(uv.x), __uint_as_float(uv.y), __uint_as_float(ti.x));
           pb.hit_inst[r] = ti.y;
         },
-        &cnt, world[threadIdx.x >> 5]);
+        &cnt, world[threadIdx.x >> 5], &entries[0][threadIdx.x]);
   }
   if (st) atomicOr(pb.status, st);
   if (kCount) {  // counters[kTraceCounterSlots * bounce + 0..10]: see nb_pathtracer_trace_counters
@@ -1809,6 +1843,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(P
   for (uint32_t i = threadIdx.x; i < wt.n_scenes; i += blockDim.x) scenes[i] = wt.scenes[i];
   __syncthreads();
   __shared__ float world[kTraceWarps][kWorldFloats];
+    __shared__ uint2 entries[kSharedEntries][kTraceThreads];
   const uint32_t st = trace_refill<true, false>(
       sq.fetch + bounce, n,
       [&](uint32_t r, V3& o, V3& d, uint32_t& sidx) {
@@ -1825,7 +1860,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(P
           pb.radiance[id] = make_float4(rr.x + c.x, rr.y + c.y, rr.z + c.z, 0.0f);
         }
       },
-      nullptr, world[threadIdx.x >> 5]);
+      nullptr, world[threadIdx.x >> 5], &entries[0][threadIdx.x]);
   if (st) atomicOr(pb.status, st);
 }
 
