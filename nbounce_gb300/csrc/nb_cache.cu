@@ -83,6 +83,11 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 __device__ __forceinline__ float relu(float x) { return fmaxf(x, 0.0f); }
+// pack2(relu(lo), relu(hi)): rounding and ReLU commute (both turn NaN into 0)
+__device__ __forceinline__ uint32_t pack2_relu(float lo, float hi) {
+  const __nv_bfloat162 v = __hmax2(__floats2bfloat162_rn(lo, hi), __floats2bfloat162_rn(0.0f, 0.0f));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 // x where the bf16 activation h (low or high half of u) is positive, else 0
 __device__ __forceinline__ float gate_lo(float x, uint32_t u) {
   return __bfloat162float(__ushort_as_bfloat16((unsigned short)(u & 0xFFFFu))) > 0.0f ? x : 0.0f;
@@ -401,11 +406,42 @@ __device__ __forceinline__ void tc_ld64(uint32_t taddr, float (&v)[64]) {
   for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Rows row0 .. row0 + 31 (one warp's) of encoded FP32 inputs X, rounded to BF16, into rows
+// 32 w .. 32 w + 31 of a canonical operand tile; rows from `end` on are zero.  A warp instruction reads
+// 128 contiguous bytes of each of 8 rows (whole sectors, one 256-bit load per lane where X is 32-byte
+// aligned) and stores 128 contiguous bytes per 8 lanes (no bank conflicts).
+__device__ __forceinline__ void stage_rows(const float* __restrict__ X, bool aligned, uint32_t row0, uint32_t end,
+                                           unsigned char* tile, uint32_t w) {
+  const uint32_t lane = threadIdx.x & 31u, r = lane & 7u;
+  float x[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t row = row0 + 8u * (i >> 1) + r, c = (lane >> 3) + 4u * (i & 1);
+    const float* p = X + (size_t)row * 64 + 8u * c;
+    if (row >= end) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[i][k] = 0.0f;
+    } else if (aligned) {
+      asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=f"(x[i][0]), "=f"(x[i][1]), "=f"(x[i][2]), "=f"(x[i][3]), "=f"(x[i][4]), "=f"(x[i][5]), "=f"(x[i][6]),
+            "=f"(x[i][7])
+          : "l"(p));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[i][k] = __ldg(p + k);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    *reinterpret_cast<uint4*>(tile + canon_off(32u * w + 8u * (i >> 1) + r, 8u * ((lane >> 3) + 4u * (i & 1)))) =
+        make_uint4(pack2(x[i][0], x[i][1]), pack2(x[i][2], x[i][3]), pack2(x[i][4], x[i][5]), pack2(x[i][6], x[i][7]));
+}
+
 // kQueries: the rows are a wave's cache queries (encoded here; results go to radiance / tail);
-// else rows of encoded inputs X (bf16 [n][64]) with results in out[n][3].
+// else rows of encoded inputs X (FP32 [n][64], rounded to BF16 here) with results in out[n][3].
 template <bool kQueries>
 __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __restrict__ W,
-                                                                  const bf16* __restrict__ X,
+                                                                  const float* __restrict__ X,
                                                                   const CacheQuery* __restrict__ queries,
                                                                   const uint32_t* __restrict__ n_dev, uint32_t n_host,
                                                                   CacheBounds bounds, float* __restrict__ out,
@@ -422,6 +458,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __
   unsigned char* act = smem_tc + kTcWBytes + 2u * wg * kTcActBytes;
   const uint32_t mbar = saddr(&mbar_slot[2 * wg]);
   const uint32_t n = kQueries ? min(*n_dev, n_host) : n_host;
+  const bool x_aligned = !kQueries && (reinterpret_cast<uintptr_t>(X) & 31u) == 0;
 
   // weights into the canonical layout: row r of layer l = global row 64 l + r.  Consecutive
   // threads take consecutive rows of one 16-byte column chunk, so each quarter-warp stores 128
@@ -473,31 +510,29 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __
     V3 fac[2];
 #pragma unroll
     for (uint32_t j = 0; j < 2; ++j) {
-      const uint32_t row = (4u * q + 2u * wg + j) * kTcRows + tid;
+      const uint32_t group0 = (4u * q + 2u * wg + j) * kTcRows, row = group0 + tid;
+      unsigned char* a = act + j * kTcActBytes;
       T[j] = make_float4(0.f, 0.f, 0.f, 0.f);
       fac[j] = V3{0.0f, 0.0f, 0.0f};
-      uint4 ch[8];
-      if (row < n) {
-        if (kQueries) {
-          const CacheQuery qr = queries[row];
-          tag[j] = qr.f.tag;
-          T[j] = qr.T;
-          fac[j] = cache_factor(qr.f);
-          float f[64];
-          cache_encode(qr.f, bounds, f);
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-            ch[c] = make_uint4(pack2(f[8 * c], f[8 * c + 1]), pack2(f[8 * c + 2], f[8 * c + 3]),
-                               pack2(f[8 * c + 4], f[8 * c + 5]), pack2(f[8 * c + 6], f[8 * c + 7]));
-        } else {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) ch[c] = __ldg(reinterpret_cast<const uint4*>(X + (size_t)row * 64) + c);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) ch[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (!kQueries) {
+        stage_rows(X, x_aligned, group0 + 32u * (warp & 3u), n, a, warp & 3u);
+        continue;
       }
-      unsigned char* a = act + j * kTcActBytes;
+      uint4 ch[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) ch[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < n) {
+        const CacheQuery qr = queries[row];
+        tag[j] = qr.f.tag;
+        T[j] = qr.T;
+        fac[j] = cache_factor(qr.f);
+        float f[64];
+        cache_encode(qr.f, bounds, f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          ch[c] = make_uint4(pack2(f[8 * c], f[8 * c + 1]), pack2(f[8 * c + 2], f[8 * c + 3]),
+                             pack2(f[8 * c + 4], f[8 * c + 5]), pack2(f[8 * c + 6], f[8 * c + 7]));
+      }
 #pragma unroll
       for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(a + canon_off(tid, 8u * c)) = ch[c];
     }
@@ -508,6 +543,12 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __
     if (tid == 0) {
       issue(0, 0);
       issue(1, 0);
+      // the next round's rows come into L2 behind this round's layers
+      const uint32_t next = (4u * (q + gridDim.x) + 2u * wg) * kTcRows;
+      if (!kQueries && x_aligned && next < n)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(X + (size_t)next * 64),
+                     "r"(min(n - next, 2u * kTcRows) * 256u)
+                     : "memory");
     }
 #pragma unroll 1
     for (int l = 0; l < 6 && !failed; ++l) {
@@ -524,8 +565,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             *reinterpret_cast<uint4*>(a + canon_off(tid, 8u * c)) =
-                make_uint4(pack2(relu(v[8 * c]), relu(v[8 * c + 1])), pack2(relu(v[8 * c + 2]), relu(v[8 * c + 3])),
-                           pack2(relu(v[8 * c + 4]), relu(v[8 * c + 5])), pack2(relu(v[8 * c + 6]), relu(v[8 * c + 7])));
+                make_uint4(pack2_relu(v[8 * c], v[8 * c + 1]), pack2_relu(v[8 * c + 2], v[8 * c + 3]),
+                           pack2_relu(v[8 * c + 4], v[8 * c + 5]), pack2_relu(v[8 * c + 6], v[8 * c + 7]));
           fence_async_smem();
         } else {
           // every lane of every warp runs the (warp-collective) accumulator load; only rows
@@ -833,9 +874,12 @@ __host__ __device__ constexpr uint32_t tc_idesc2(uint32_t M, uint32_t N, bool a_
 // MN-major operand (features x rows): leading byte offset G (between 8-row groups, along K),
 // stride byte offset 128 B (between 8-feature chunks, along M or N).
 
+// kRaw: the rows are the caller's, X FP32 [n][64] and Y FP32 [n][3]; else a frame's records, X BF16
+// [n][64] and Y float4 [n] (.w = 0: no target).
+template <bool kRaw>
 __global__ void __launch_bounds__(128, 1) k_cache_grad_tc(const unsigned char* __restrict__ stage,
-                                                          const bf16* __restrict__ X,
-                                                          const float4* __restrict__ Y,
+                                                          const void* __restrict__ X,
+                                                          const void* __restrict__ Y,
                                                           const uint32_t* __restrict__ n_dev, uint32_t n_host,
                                                           uint32_t row0, uint32_t rows_per_step, float clip,
                                                           float* __restrict__ part_dw, float* __restrict__ part_loss,
@@ -872,14 +916,16 @@ __global__ void __launch_bounds__(128, 1) k_cache_grad_tc(const unsigned char* _
                    : "memory");
     }
   }
-  // this thread's input row
-  {
+  // the input rows
+  if (kRaw) {
+    const float* x = static_cast<const float*>(X);
+    stage_rows(x, (reinterpret_cast<uintptr_t>(x) & 31u) == 0, row - tid + 32u * warp, end, H, warp);
+  } else {
     const bool live = row < end;
+    const uint4* x = reinterpret_cast<const uint4*>(static_cast<const bf16*>(X) + (size_t)row * 64);
 #pragma unroll
-    for (uint32_t c = 0; c < 8; ++c) {
-      const uint4 v = live ? __ldg(reinterpret_cast<const uint4*>(X + (size_t)row * 64) + c) : make_uint4(0u, 0u, 0u, 0u);
-      *reinterpret_cast<uint4*>(H + canon_off(tid, 8u * c)) = v;
-    }
+    for (uint32_t c = 0; c < 8; ++c)
+      *reinterpret_cast<uint4*>(H + canon_off(tid, 8u * c)) = live ? __ldg(x + c) : make_uint4(0u, 0u, 0u, 0u);
   }
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
@@ -942,15 +988,21 @@ __global__ void __launch_bounds__(128, 1) k_cache_grad_tc(const unsigned char* _
 #pragma unroll
       for (uint32_t c = 0; c < 8; ++c)
         *reinterpret_cast<uint4*>(h + canon_off(tid, 8u * c)) =
-            make_uint4(pack2(relu(v[8 * c]), relu(v[8 * c + 1])), pack2(relu(v[8 * c + 2]), relu(v[8 * c + 3])),
-                       pack2(relu(v[8 * c + 4]), relu(v[8 * c + 5])), pack2(relu(v[8 * c + 6]), relu(v[8 * c + 7])));
+            make_uint4(pack2_relu(v[8 * c], v[8 * c + 1]), pack2_relu(v[8 * c + 2], v[8 * c + 3]),
+                       pack2_relu(v[8 * c + 4], v[8 * c + 5]), pack2_relu(v[8 * c + 6], v[8 * c + 7]));
     } else {
       // output layer: dL/dp = 2 (p - y) / (p^2 + 0.01) with the denominator held constant
       float v[16];
       tc_ld16(d_layer + lane_base, v);
       float gz[3] = {0.0f, 0.0f, 0.0f}, lsum = 0.0f;
       if (row < end) {
-        const float4 y4 = __ldg(Y + row);
+        float4 y4;
+        if (kRaw) {
+          const float* y = static_cast<const float*>(Y) + 3 * (size_t)row;
+          y4 = make_float4(__ldg(y), __ldg(y + 1), __ldg(y + 2), 1.0f);
+        } else {
+          y4 = __ldg(static_cast<const float4*>(Y) + row);
+        }
         if (y4.w != 0.0f) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
@@ -1074,25 +1126,44 @@ __global__ void __launch_bounds__(256) k_cache_adam(float* __restrict__ w, bf16*
                                                     uint32_t row0, uint32_t rows_per_step, AdamArgs args,
                                                     float* __restrict__ grad_out, float* __restrict__ loss_out) {
   __shared__ float red[8][kAdamParams];
+  __shared__ float loss_sh[256];
   const uint32_t n_total = n_dev ? *n_dev : n_host;
   const uint32_t rows = n_total > row0 ? min(n_total - row0, rows_per_step) : 0u;
   const uint32_t lane = threadIdx.x & 31u, grp = threadIdx.x >> 5;
   const uint32_t p = blockIdx.x * kAdamParams + lane;
   const uint32_t parts = (rows + kGradRows - 1) / kGradRows;
   const float scale = rows ? 1.0f / (3.0f * (float)rows) : 0.0f;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && loss_out) {
+  if (blockIdx.x == gridDim.x - 1 && loss_out) {  // in order, from shared memory
     float s = 0.0f;
-    for (uint32_t c = 0; c < parts; ++c) s += part_loss[c];
-    *loss_out = s * scale;
+    for (uint32_t c = 0; c < parts; c += blockDim.x) {
+      loss_sh[threadIdx.x] = c + threadIdx.x < parts ? part_loss[c + threadIdx.x] : 0.0f;
+      __syncthreads();
+      const uint32_t m = min(parts - c, (uint32_t)blockDim.x);
+      if (threadIdx.x == 0)
+        for (uint32_t k = 0; k < m; ++k) s += loss_sh[k];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss_out = s * scale;
   }
   float a0 = 0.0f, a1 = 0.0f;
   if (p < (uint32_t)kMlpParams) {
+    const float* d = part_dw + p;
     uint32_t c = grp;
-    for (; c + 8 < parts; c += 16) {
-      a0 += part_dw[(size_t)c * kMlpParams + p];
-      a1 += part_dw[(size_t)(c + 8) * kMlpParams + p];
+    for (; c + 56 < parts; c += 64) {  // eight partials in flight, added in the order of the loop below
+      float x[8];
+#pragma unroll
+      for (uint32_t k = 0; k < 8; ++k) x[k] = __ldcg(d + (size_t)(c + 8 * k) * kMlpParams);
+#pragma unroll
+      for (uint32_t k = 0; k < 8; k += 2) {
+        a0 += x[k];
+        a1 += x[k + 1];
+      }
     }
-    if (c < parts) a0 += part_dw[(size_t)c * kMlpParams + p];
+    for (; c + 8 < parts; c += 16) {
+      a0 += __ldcg(d + (size_t)c * kMlpParams);
+      a1 += __ldcg(d + (size_t)(c + 8) * kMlpParams);
+    }
+    if (c < parts) a0 += __ldcg(d + (size_t)c * kMlpParams);
   }
   red[grp][lane] = a0 + a1;
   __syncthreads();
@@ -1302,7 +1373,14 @@ struct nb_cache {
   nbd::bf16* web = nullptr;
   float* m = nullptr;
   float* v = nullptr;
-  uint32_t* status = nullptr;  // tensor-core wait timeouts of nb_cache_infer / training
+  // Tensor-core wait timeouts of nb_cache_infer / training, and the loss of a caller's batch: in
+  // page-locked host memory that the kernels write (the status only on a timeout), so that a call
+  // that reports them needs a stream synchronisation and no copies
+  struct Report {
+    uint32_t status;
+    float loss;
+  };
+  Report* report = nullptr;
   unsigned char* wstage = nullptr;  // training weight image (k_cache_grad_tc), kept by k_cache_adam
   float* part_dw = nullptr;
   float* part_loss = nullptr;
@@ -1366,7 +1444,10 @@ int set_smem_limits() {
       e = cudaFuncSetAttribute(nbd::k_cache_infer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)nbd::kTcSmem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(nbd::k_cache_grad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(nbd::k_cache_grad_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)nbd::kTrSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(nbd::k_cache_grad_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)nbd::kTrSmem);
     rc = e == cudaSuccess ? NB_OK : cuda_fail(e, "cudaFuncSetAttribute(cache kernels)");
   });
@@ -1440,16 +1521,18 @@ int grid_for(size_t n, int threads, int sms) {
 
 // one optimiser step (update) or gradient evaluation over rows [row0, row0 + rows_per_step)
 // of (X, Y); n_dev (device row count) or n_host bounds the rows
-cudaError_t train_launch(nb_cache* c, const nbd::bf16* X, const float4* Y, const uint32_t* n_dev, uint32_t n_host,
+// raw: X and Y are the caller's FP32 rows and targets (tcgen05 path only)
+cudaError_t train_launch(nb_cache* c, const void* X, const void* Y, bool raw, const uint32_t* n_dev, uint32_t n_host,
                          uint32_t row0, uint32_t rows_per_step, bool update, float* grad_out, float* loss_out,
                          cudaStream_t st) {
   const uint32_t ctas = (rows_per_step + nbd::kGradRows - 1) / nbd::kGradRows;
   if (c->cfg.tensor_path == NB_CACHE_TCGEN05)
-    nbd::k_cache_grad_tc<<<ctas, 128, nbd::kTrSmem, st>>>(c->wstage, X, Y, n_dev, n_host, row0, rows_per_step,
-                                                          c->cfg.grad_clip, c->part_dw, c->part_loss, c->status);
+    (raw ? nbd::k_cache_grad_tc<true> : nbd::k_cache_grad_tc<false>)<<<ctas, 128, nbd::kTrSmem, st>>>(
+        c->wstage, X, Y, n_dev, n_host, row0, rows_per_step, c->cfg.grad_clip, c->part_dw, c->part_loss, &c->report->status);
   else
-    nbd::k_cache_grad<<<ctas, 256, nbd::kGradSmem, st>>>(c->wb, X, Y, n_dev, n_host, row0, rows_per_step,
-                                                         c->cfg.grad_clip, c->part_dw, c->part_loss);
+    nbd::k_cache_grad<<<ctas, 256, nbd::kGradSmem, st>>>(c->wb, static_cast<const nbd::bf16*>(X),
+                                                         static_cast<const float4*>(Y), n_dev, n_host, row0,
+                                                         rows_per_step, c->cfg.grad_clip, c->part_dw, c->part_loss);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   nbd::AdamArgs a{};
@@ -1603,7 +1686,7 @@ int cache_wave_train(nb_cache* c, uint32_t n_paths, int sms, cudaStream_t st) {
   const uint32_t steps = c->cfg.train_steps;
   const uint32_t per = steps ? (c->cfg.train_records + steps - 1) / steps : 0;
   for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k)
-    e = train_launch(c, c->X, c->Y, c->counters + 2, 0, k * per, per, c->cfg.learning_rate > 0.0f, nullptr,
+    e = train_launch(c, c->X, c->Y, false, c->counters + 2, 0, k * per, per, c->cfg.learning_rate > 0.0f, nullptr,
                      c->losses + k, st);
   if (e != cudaSuccess) return cuda_fail(e, "cache wave launch");
   c->last_steps = steps;
@@ -1654,7 +1737,7 @@ int nb_cache_create(const nb_cache_config* cfg, nb_cache** out) {
   nb_cache* h = new (std::nothrow) nb_cache();
   if (!h) return fail(NB_ERR_OOM, "host allocation failed");
   h->cfg = c;
-  void* p[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  void* p[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   int rc = NB_OK;
   for (int k = 0; k < 6 && !rc; ++k)
     rc = h->arena.alloc(kMlpParams * ((k == 1 || k == 3) ? sizeof(nbd::bf16) : sizeof(float)), &p[k]);
@@ -1664,8 +1747,11 @@ int nb_cache_create(const nb_cache_config* cfg, nb_cache** out) {
   h->web = (nbd::bf16*)p[3];
   h->m = (float*)p[4];
   h->v = (float*)p[5];
-  if (!rc) rc = h->arena.alloc(sizeof(uint32_t), &p[6]);
-  h->status = (uint32_t*)p[6];
+  if (!rc) {
+    const cudaError_t e = cudaHostAlloc((void**)&h->report, sizeof(nb_cache::Report), cudaHostAllocPortable);
+    if (e != cudaSuccess) rc = cuda_fail(e, "cudaHostAlloc(cache report)");
+    else *h->report = nb_cache::Report{0, 0.0f};
+  }
   void* stage = nullptr;
   if (!rc) rc = h->arena.alloc(nbd::kTrStage, &stage);
   h->wstage = (unsigned char*)stage;
@@ -1680,6 +1766,7 @@ int nb_cache_create(const nb_cache_config* cfg, nb_cache** out) {
   }
   if (rc) {
     h->arena.release();
+    if (h->report) cudaFreeHost(h->report);
     delete h;
     return rc;
   }
@@ -1693,6 +1780,7 @@ void nb_cache_destroy(nb_cache* c) {
   c->arena.release();
   c->wave.release();
   c->scratch.release();
+  cudaFreeHost(c->report);
   delete c;
 }
 
@@ -1748,25 +1836,25 @@ int nb_cache_infer(nb_cache* c, const float* enc, size_t n, float* out, void* st
   if (n > (1u << 30)) return fail(NB_ERR_INVALID_ARG, "too many rows");
   std::lock_guard<std::mutex> lk(c->mu);
   int rc = set_smem_limits();
-  if (rc || (rc = ensure_scratch(c, n))) return rc;
+  if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int sms = sm_count();
-  nbd::k_to_bf16<<<grid_for(n * 64, 256, sms), 256, 0, st>>>(enc, c->sx, n * 64);
   if (c->cfg.tensor_path == NB_CACHE_TCGEN05) {
-    NB_CUDA(cudaMemsetAsync(c->status, 0, sizeof(uint32_t), st), "cudaMemsetAsync");
+    c->report->status = 0;
     const size_t rounds = (n + 4 * nbd::kTcRows - 1) / (4 * nbd::kTcRows);
     nbd::k_cache_infer_tc<false><<<(unsigned)std::min<size_t>(rounds, 2 * (size_t)sms), nbd::kTcThreads,
-                                   nbd::kTcSmem, st>>>(c->wb, c->sx, nullptr, nullptr, (uint32_t)n, c->bounds, out,
-                                                       nullptr, nullptr, c->status);
+                                   nbd::kTcSmem, st>>>(c->wb, enc, nullptr, nullptr, (uint32_t)n, c->bounds, out,
+                                                       nullptr, nullptr, &c->report->status);
   } else {
+    if ((rc = ensure_scratch(c, n))) return rc;
+    nbd::k_to_bf16<<<grid_for(n * 64, 256, sms), 256, 0, st>>>(enc, c->sx, n * 64);
     nbd::k_cache_infer_rows<<<std::min<size_t>((n + 255) / 256, 2 * (size_t)sms), 256, nbd::kInferSmem, st>>>(
         c->wb, c->sx, (uint32_t)n, out);
   }
   NB_CUDA(cudaGetLastError(), "cache infer launch");
   if (c->cfg.tensor_path == NB_CACHE_TCGEN05) {
-    uint32_t status = 0;
-    NB_CUDA(cudaMemcpyAsync(&status, c->status, sizeof(status), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
     NB_CUDA(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+    const uint32_t status = *(volatile uint32_t*)&c->report->status;
     if (status & nbd::kStatusCacheTimeout)
       return fail(NB_ERR_TIMEOUT, "tensor-core wait timed out (layer %u)", (status >> 16) - 1u);
   }
@@ -1780,25 +1868,26 @@ static int rows_op(nb_cache* c, const float* enc, const float* target, size_t n,
   if (n > (1u << 24)) return fail(NB_ERR_INVALID_ARG, "batch larger than 2^24 rows");
   std::lock_guard<std::mutex> lk(c->mu);
   int rc = set_smem_limits();
-  if (rc || (rc = ensure_scratch(c, n))) return rc;
+  const bool tc = c->cfg.tensor_path == NB_CACHE_TCGEN05;
+  if (rc || (!tc && (rc = ensure_scratch(c, n)))) return rc;
   const uint32_t ctas = (uint32_t)((n + nbd::kGradRows - 1) / nbd::kGradRows);
-  if ((rc = ensure_parts(c, ctas)) || (rc = ensure_losses(c, 1))) return rc;
+  if ((rc = ensure_parts(c, ctas))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int sms = sm_count();
-  const bool tc = c->cfg.tensor_path == NB_CACHE_TCGEN05;
-  cudaError_t e = tc ? cudaMemsetAsync(c->status, 0, sizeof(uint32_t), st) : cudaSuccess;
-  if (e == cudaSuccess) {
+  cudaError_t e = cudaSuccess;
+  c->report->status = 0;
+  if (e == cudaSuccess && !tc) {
     nbd::k_to_bf16<<<grid_for(n * 64, 256, sms), 256, 0, st>>>(enc, c->sx, n * 64);
     nbd::k_targets<<<grid_for(n, 256, sms), 256, 0, st>>>(target, c->sy, n);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)
-    e = train_launch(c, c->sx, c->sy, nullptr, (uint32_t)n, 0, (uint32_t)n, update, grad, c->losses, st);
-  if (e == cudaSuccess && loss) e = cudaMemcpyAsync(loss, c->losses, sizeof(float), cudaMemcpyDeviceToHost, st);
-  uint32_t status = 0;
-  if (e == cudaSuccess && tc) e = cudaMemcpyAsync(&status, c->status, sizeof(status), cudaMemcpyDeviceToHost, st);
+    e = train_launch(c, tc ? (const void*)enc : c->sx, tc ? (const void*)target : c->sy, tc, nullptr, (uint32_t)n, 0,
+                     (uint32_t)n, update, grad, &c->report->loss, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "cache training launch");
+  if (loss) *loss = *(volatile float*)&c->report->loss;
+  const uint32_t status = *(volatile uint32_t*)&c->report->status;
   if (status & nbd::kStatusCacheTimeout) return fail(NB_ERR_TIMEOUT, "tensor-core wait timed out in training");
   return NB_OK;
 }
