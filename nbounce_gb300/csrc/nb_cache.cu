@@ -298,28 +298,31 @@ __global__ void __launch_bounds__(256, 2) k_cache_infer_queries(const bf16* __re
 
 // ---- inference on the 5th-generation tensor cores (tcgen05) ------------------------------
 //
-// A CTA is two warpgroups of 4 warps; each warpgroup keeps two groups of 128 rows in flight,
-// so an SM (2 CTAs) runs 8 independent layer chains and one chain's MMA round trip hides
-// behind the others' epilogues.  The MMA operands sit in shared memory in the no-swizzle
-// K-major canonical layout of tcgen05.mma: 8-row x 16-byte core matrices of 128 B, the core
-// matrices of one 8-row group along K contiguous (leading byte offset 128 B), 8-row groups
-// 1 KB apart (stride byte offset 1 KB).  Each group's accumulator (128 lanes x 64 FP32 columns)
-// lives in tensor memory.  Per layer and group the warpgroup's first thread issues four
-// K = 16 MMAs and commits them to the group's mbarrier; once they completed, the warps read
-// their 32 accumulator rows (tcgen05.ld), apply ReLU, pack to BF16 and overwrite the group's
-// operand with the next layer's (the MMA that read it is done).  The warp-collective
-// (.sync.aligned) tcgen05 instructions - alloc, ld, dealloc - run on whole converged warps.
-// Waits poll the mbarrier a bounded number of times: on a timeout the warpgroup raises
-// kStatusCacheTimeout (bits 16.. = 1 + the layer it waited for) and stops; the CTA frees its
+// One CTA per SM, four warpgroups, each running groups of 128 rows (thread = row = TMEM lane) through
+// the layers on its own, so four layer chains hide each other's latency.  A layer is D = A W^T with the
+// weights in shared memory (no-swizzle K-major canonical layout of tcgen05.mma: 8-row x 16-byte core
+// matrices of 128 B, the core matrices of one 8-row group along K contiguous, leading byte offset
+// 128 B, 8-row groups 1 KB apart, stride byte offset 1 KB) and the activations A and the accumulator
+// D in tensor memory: a warpgroup has 64 FP32 columns of D and 32 columns of A (two BF16 per column).
+// The warpgroup's first thread issues four K = 16 MMAs and commits them to the warpgroup's mbarrier;
+// then the warps read their accumulator rows (tcgen05.ld), apply ReLU, round to BF16 and store the
+// next layer's A (tcgen05.st).  Activations never pass through shared memory: with the operand there
+// (8 chains per SM) its stores and the MMAs' reads of it took 51% of the shared-memory pipe, all
+// requests 65%, and a million rows 101 us; this way they take 74 us (the rows' bytes 38 us, the
+// rest the latency of the chains: an MMA round trip, two barriers, the accumulator's load and the
+// operand's store per layer).  The caller's rows are loaded one group ahead, behind the
+// layers of the group before.  The warp-collective (.sync.aligned) tcgen05 instructions run on whole
+// converged warps.  Waits poll the mbarrier a bounded number of times: on a timeout the warpgroup
+// raises kStatusCacheTimeout (bits 16.. = 1 + the layer it waited for) and stops; the CTA frees its
 // TMEM before it exits.
 
 constexpr int kTcRows = 128;                                   // rows per group (= TMEM lanes)
-constexpr int kTcThreads = 256;                                // two warpgroups
-constexpr uint32_t kTcCols = 256;                              // TMEM columns: 64 per group, 4 groups
+constexpr int kTcGroups = 4;                                   // warpgroups of a CTA
+constexpr int kTcThreads = 128 * kTcGroups;
+constexpr uint32_t kTcCols = 128 * kTcGroups;                  // TMEM columns: 64 D + 32 A (+ 32) each
 constexpr uint32_t kTcLayerBytes = 8192;                       // one 64 x 64 layer, canonical
 constexpr size_t kTcWBytes = 5 * kTcLayerBytes + 2048;         // + the 16 x 64 output layer
-constexpr size_t kTcActBytes = (size_t)kTcRows * 64 * sizeof(bf16);  // 16 KB per group operand
-constexpr size_t kTcSmem = kTcWBytes + 4 * kTcActBytes;        // 108,544 B (2 CTAs per SM)
+constexpr size_t kTcSmem = kTcWBytes;
 constexpr uint32_t kTcWaitLimit = 1u << 22;                    // mbarrier polls per wait
 constexpr uint32_t kStatusCacheTimeout = 1u << 8;
 
@@ -345,6 +348,15 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a, uint64_t b, 
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// the same with A in tensor memory
+__device__ __forceinline__ void tc_mma_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void tc_commit(uint32_t mbar) {
@@ -379,6 +391,9 @@ __device__ __forceinline__ bool wg_barrier_or(uint32_t wg, bool pred) {
       : "memory");
   return out != 0;
 }
+__device__ __forceinline__ void wg_barrier(uint32_t wg) {
+  asm volatile("bar.sync %0, 128;\n" ::"r"(1u + wg) : "memory");
+}
 // 16 consecutive FP32 accumulator columns of this thread's TMEM lane
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
@@ -405,6 +420,28 @@ __device__ __forceinline__ void tc_ld64(uint32_t taddr, float (&v)[64]) {
 #pragma unroll
   for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
+
+// 32 consecutive FP32 accumulator columns of this thread's TMEM lane
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
+  uint32_t r[32];
+  __syncwarp();  // warp-collective
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+               "tcgen05.wait::ld.sync.aligned;\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+               : "r"(taddr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+// 16 consecutive 32-bit columns of this thread's TMEM lane (32 BF16 of an A operand); tc_wait_st before
+// anything reads them
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  __syncwarp();  // warp-collective
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::"r"(taddr),
+               "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
 // Rows row0 .. row0 + 31 (one warp's) of encoded FP32 inputs X, rounded to BF16, into rows
 // 32 w .. 32 w + 31 of a canonical operand tile; rows from `end` on are zero.  A warp instruction reads
@@ -437,10 +474,27 @@ __device__ __forceinline__ void stage_rows(const float* __restrict__ X, bool ali
         make_uint4(pack2(x[i][0], x[i][1]), pack2(x[i][2], x[i][3]), pack2(x[i][4], x[i][5]), pack2(x[i][6], x[i][7]));
 }
 
+// One row of encoded FP32 inputs, 32 bytes per load where X is 32-byte aligned
+__device__ __forceinline__ void load_row(const float* __restrict__ p, bool aligned, float (&x)[64]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (aligned) {
+      // volatile: stays ahead of the layers it is to run behind
+      asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=f"(x[8 * i]), "=f"(x[8 * i + 1]), "=f"(x[8 * i + 2]), "=f"(x[8 * i + 3]), "=f"(x[8 * i + 4]),
+            "=f"(x[8 * i + 5]), "=f"(x[8 * i + 6]), "=f"(x[8 * i + 7])
+          : "l"(p + 8 * i));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[8 * i + k] = __ldg(p + 8 * i + k);
+    }
+  }
+}
+
 // kQueries: the rows are a wave's cache queries (encoded here; results go to radiance / tail);
 // else rows of encoded inputs X (FP32 [n][64], rounded to BF16 here) with results in out[n][3].
 template <bool kQueries>
-__global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __restrict__ W,
+__global__ void __launch_bounds__(kTcThreads, 1) k_cache_infer_tc(const bf16* __restrict__ W,
                                                                   const float* __restrict__ X,
                                                                   const CacheQuery* __restrict__ queries,
                                                                   const uint32_t* __restrict__ n_dev, uint32_t n_host,
@@ -449,16 +503,27 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __
                                                                   float4* __restrict__ tail,
                                                                   uint32_t* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem_tc[];
-  __shared__ __align__(8) uint64_t mbar_slot[4];
+  __shared__ __align__(8) uint64_t mbar_slot[kTcGroups];
   __shared__ uint32_t tmem_slot;
   unsigned char* Wc = smem_tc;
   const uint32_t warp = threadIdx.x >> 5, wg = threadIdx.x >> 7, tid = threadIdx.x & 127u;
-  // group j of warpgroup wg: operand at act + j * kTcActBytes, mbarrier mbar + 8 j, accumulator
-  // columns 128 wg + 64 j
-  unsigned char* act = smem_tc + kTcWBytes + 2u * wg * kTcActBytes;
-  const uint32_t mbar = saddr(&mbar_slot[2 * wg]);
+  const uint32_t mbar = saddr(&mbar_slot[wg]);
   const uint32_t n = kQueries ? min(*n_dev, n_host) : n_host;
-  const bool x_aligned = !kQueries && (reinterpret_cast<uintptr_t>(X) & 31u) == 0;
+  const uint32_t groups = (n + kTcRows - 1) / kTcRows, stride = gridDim.x * kTcGroups;
+  const bool aligned = !kQueries && (reinterpret_cast<uintptr_t>(X) & 31u) == 0;
+  // the groups are dealt to the CTAs first, so that few groups use many SMs
+  uint32_t group = wg * gridDim.x + blockIdx.x;
+  float x[64];  // this thread's next row (!kQueries)
+  auto fetch = [&](uint32_t g) {
+    const uint32_t row = g * kTcRows + tid;
+    if (g < groups && row < n) {
+      load_row(X + (size_t)row * 64, aligned, x);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 64; ++k) x[k] = 0.0f;
+    }
+  };
+  if (!kQueries) fetch(group);
 
   // weights into the canonical layout: row r of layer l = global row 64 l + r.  Consecutive
   // threads take consecutive rows of one 16-byte column chunk, so each quarter-warp stores 128
@@ -469,7 +534,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __
         __ldg(reinterpret_cast<const uint4*>(W) + 8u * row + c);
   }
   if (threadIdx.x == 0) {
-    for (uint32_t k = 0; k < 4; ++k)
+    for (uint32_t k = 0; k < (uint32_t)kTcGroups; ++k)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(&mbar_slot[k])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -484,130 +549,94 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_cache_infer_tc(const bf16* __
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_slot + 128u * wg;            // this warpgroup's two accumulators
+  const uint32_t d_tmem = tmem_slot + 128u * wg, a_tmem = d_tmem + 64u;
   const uint32_t lane_base = (32u * (warp & 3u)) << 16;  // this warp's 32 TMEM lanes
-  uint32_t phase[2] = {0u, 0u};
-  uint32_t fail_layer = 0;
+  uint32_t phase = 0, fail_layer = 0;
   bool failed = false;
 
-  // layer l of group j: four K = 16 MMAs into the group's 64 accumulator columns
-  auto issue = [&](uint32_t j, int l) {
-    const uint32_t a_base = saddr(act + j * kTcActBytes);
-    const uint32_t b_base = saddr(Wc + l * kTcLayerBytes);
-    const uint32_t idesc = tc_idesc(kTcRows, l < 5 ? 64u : 16u);
+  for (; group < groups && !failed; group += stride) {
+    const uint32_t row = group * kTcRows + tid;
+    uint32_t tag = 0;
+    float4 T = make_float4(0.f, 0.f, 0.f, 0.f);
+    V3 fac{0.0f, 0.0f, 0.0f};
+    if (kQueries) {
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k)
-      tc_mma(tmem + 64u * j, tc_desc(a_base + 256u * k), tc_desc(b_base + 256u * k), idesc, k);
-    tc_commit(mbar + 8u * j);
-  };
-
-  const uint32_t groups = (n + kTcRows - 1) / kTcRows;
-  // round q covers row groups 4 q .. 4 q + 3 (warpgroup wg takes 4 q + 2 wg + j); rounds are
-  // dealt to the CTAs round-robin
-  for (uint32_t q = blockIdx.x; 4u * q + 2u * wg < groups && !failed; q += gridDim.x) {
-    uint32_t tag[2] = {0u, 0u};
-    float4 T[2];
-    V3 fac[2];
-#pragma unroll
-    for (uint32_t j = 0; j < 2; ++j) {
-      const uint32_t group0 = (4u * q + 2u * wg + j) * kTcRows, row = group0 + tid;
-      unsigned char* a = act + j * kTcActBytes;
-      T[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      fac[j] = V3{0.0f, 0.0f, 0.0f};
-      if (!kQueries) {
-        stage_rows(X, x_aligned, group0 + 32u * (warp & 3u), n, a, warp & 3u);
-        continue;
-      }
-      uint4 ch[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) ch[c] = make_uint4(0u, 0u, 0u, 0u);
+      for (int k = 0; k < 64; ++k) x[k] = 0.0f;
       if (row < n) {
         const CacheQuery qr = queries[row];
-        tag[j] = qr.f.tag;
-        T[j] = qr.T;
-        fac[j] = cache_factor(qr.f);
-        float f[64];
-        cache_encode(qr.f, bounds, f);
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          ch[c] = make_uint4(pack2(f[8 * c], f[8 * c + 1]), pack2(f[8 * c + 2], f[8 * c + 3]),
-                             pack2(f[8 * c + 4], f[8 * c + 5]), pack2(f[8 * c + 6], f[8 * c + 7]));
+        tag = qr.f.tag;
+        T = qr.T;
+        fac = cache_factor(qr.f);
+        cache_encode(qr.f, bounds, x);
       }
+    }
 #pragma unroll
-      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(a + canon_off(tid, 8u * c)) = ch[c];
+    for (int h = 0; h < 2; ++h) {
+      uint32_t r[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) r[k] = pack2(x[32 * h + 2 * k], x[32 * h + 2 * k + 1]);
+      tc_st16(a_tmem + lane_base + 16u * h, r);
     }
-    fence_async_smem();
-    tc_fence_before();
-    wg_barrier_or(wg, false);
-    tc_fence_after();
-    if (tid == 0) {
-      issue(0, 0);
-      issue(1, 0);
-      // the next round's rows come into L2 behind this round's layers
-      const uint32_t next = (4u * (q + gridDim.x) + 2u * wg) * kTcRows;
-      if (!kQueries && x_aligned && next < n)
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(X + (size_t)next * 64),
-                     "r"(min(n - next, 2u * kTcRows) * 256u)
-                     : "memory");
-    }
+    if (!kQueries) fetch(group + stride);
 #pragma unroll 1
-    for (int l = 0; l < 6 && !failed; ++l) {
-#pragma unroll
-      for (uint32_t j = 0; j < 2; ++j) {
-        const bool ok = mbar_wait(mbar + 8u * j, phase[j]);
-        phase[j] ^= 1u;
+    for (int l = 0; l < 6; ++l) {
+      tc_wait_st();
+      tc_fence_before();
+      wg_barrier(wg);  // the warps' rows of A are written, D is read
+      if (tid == 0) {
         tc_fence_after();
-        const uint32_t t_row = tmem + 64u * j + lane_base;
-        if (l < 5) {
-          unsigned char* a = act + j * kTcActBytes;  // its MMA is complete: overwrite in place
-          float v[64];
-          tc_ld64(t_row, v);
+        const uint32_t b = saddr(Wc + l * kTcLayerBytes), idesc = tc_idesc(kTcRows, l < 5 ? 64u : 16u);
 #pragma unroll
-          for (int c = 0; c < 8; ++c)
-            *reinterpret_cast<uint4*>(a + canon_off(tid, 8u * c)) =
-                make_uint4(pack2_relu(v[8 * c], v[8 * c + 1]), pack2_relu(v[8 * c + 2], v[8 * c + 3]),
-                           pack2_relu(v[8 * c + 4], v[8 * c + 5]), pack2_relu(v[8 * c + 6], v[8 * c + 7]));
-          fence_async_smem();
-        } else {
-          // every lane of every warp runs the (warp-collective) accumulator load; only rows
-          // of the batch use it
-          float v[16];
-          tc_ld16(t_row, v);
-          const uint32_t row = (4u * q + 2u * wg + j) * kTcRows + tid;
-          if (!ok || row >= n) {
-          } else if (kQueries) {
-            const V3 L{fmaxf(v[0], 0.0f) * fac[j].x, fmaxf(v[1], 0.0f) * fac[j].y, fmaxf(v[2], 0.0f) * fac[j].z};
-            if (tag[j] & nb::kCacheTailBit) {
-              tail[tag[j] & ~nb::kCacheTailBit] = make_float4(L.x, L.y, L.z, 0.0f);
-            } else {
-              float4 c = radiance[tag[j]];
-              c.x = c.x + T[j].x * L.x;
-              c.y = c.y + T[j].y * L.y;
-              c.z = c.z + T[j].z * L.z;
-              radiance[tag[j]] = c;
-            }
+        for (uint32_t k = 0; k < 4; ++k)
+          tc_mma_ta(d_tmem, a_tmem + 8u * k, tc_desc(b + 256u * k), idesc, k);
+        tc_commit(mbar);
+      }
+      const bool ok = mbar_wait(mbar, phase);
+      phase ^= 1u;
+      tc_fence_after();
+      failed = wg_barrier_or(wg, !ok);
+      if (failed) {
+        fail_layer = (uint32_t)l + 1u;
+        break;
+      }
+      if (l < 5) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float v[32];
+          tc_ld32(d_tmem + lane_base + 32u * h, v);
+          uint32_t r[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) r[k] = pack2_relu(v[2 * k], v[2 * k + 1]);
+          tc_st16(a_tmem + lane_base + 16u * h, r);
+        }
+      } else {
+        // every lane of every warp runs the (warp-collective) accumulator load; only rows of the
+        // batch use it
+        float v[16];
+        tc_ld16(d_tmem + lane_base, v);
+        if (row >= n) {
+        } else if (kQueries) {
+          const V3 L{fmaxf(v[0], 0.0f) * fac.x, fmaxf(v[1], 0.0f) * fac.y, fmaxf(v[2], 0.0f) * fac.z};
+          if (tag & nb::kCacheTailBit) {
+            tail[tag & ~nb::kCacheTailBit] = make_float4(L.x, L.y, L.z, 0.0f);
           } else {
-            out[3 * (size_t)row] = v[0];
-            out[3 * (size_t)row + 1] = v[1];
-            out[3 * (size_t)row + 2] = v[2];
+            float4 c = radiance[tag];
+            c.x = c.x + T.x * L.x;
+            c.y = c.y + T.y * L.y;
+            c.z = c.z + T.z * L.z;
+            radiance[tag] = c;
           }
+        } else {
+          out[3 * (size_t)row] = v[0];
+          out[3 * (size_t)row + 1] = v[1];
+          out[3 * (size_t)row + 2] = v[2];
         }
-        tc_fence_before();
-        failed = wg_barrier_or(wg, !ok);
-        tc_fence_after();
-        if (failed) {
-          fail_layer = (uint32_t)l + 1u;
-          break;
-        }
-        if (l < 5 && tid == 0) issue(j, l + 1);
       }
     }
   }
   if (failed && tid == 0) {
     atomicOr(status, kStatusCacheTimeout | (fail_layer << 16));
-    // give outstanding MMAs a bounded chance to finish before the memory is released
-    mbar_wait(mbar, phase[0] ^ 1u);
-    mbar_wait(mbar + 8u, phase[1] ^ 1u);
+    mbar_wait(mbar, phase ^ 1u);  // give outstanding MMAs a bounded chance to finish
   }
   tc_fence_before();
   __syncthreads();
@@ -1654,7 +1683,7 @@ int cache_wave_begin(nb_cache* c, const nb_scene* scene, uint32_t n_paths, Cache
 int cache_wave_infer(nb_cache* c, const PathBatch& pb, int sms, cudaStream_t st) {
   const nbd::bf16* w = c->cfg.ema > 0.0f ? c->web : c->wb;
   if (c->cfg.tensor_path == NB_CACHE_TCGEN05)
-    nbd::k_cache_infer_tc<true><<<2 * sms, nbd::kTcThreads, nbd::kTcSmem, st>>>(
+    nbd::k_cache_infer_tc<true><<<sms, nbd::kTcThreads, nbd::kTcSmem, st>>>(
         w, nullptr, c->queries, c->counters, c->cap_paths + c->cap_slots, c->bounds, nullptr, pb.radiance, c->tail,
         pb.status);
   else
@@ -1841,8 +1870,8 @@ int nb_cache_infer(nb_cache* c, const float* enc, size_t n, float* out, void* st
   const int sms = sm_count();
   if (c->cfg.tensor_path == NB_CACHE_TCGEN05) {
     c->report->status = 0;
-    const size_t rounds = (n + 4 * nbd::kTcRows - 1) / (4 * nbd::kTcRows);
-    nbd::k_cache_infer_tc<false><<<(unsigned)std::min<size_t>(rounds, 2 * (size_t)sms), nbd::kTcThreads,
+    const size_t groups = (n + nbd::kTcRows - 1) / nbd::kTcRows;
+    nbd::k_cache_infer_tc<false><<<(unsigned)std::min<size_t>(groups, (size_t)sms), nbd::kTcThreads,
                                    nbd::kTcSmem, st>>>(c->wb, enc, nullptr, nullptr, (uint32_t)n, c->bounds, out,
                                                        nullptr, nullptr, &c->report->status);
   } else {
