@@ -624,8 +624,9 @@ static int render_samples(nb_pathtracer* pt, const nb_scene* scene, const nb_cam
   if (!scene->uploaded) return fail(NB_ERR_INVALID_ARG, "scene was built with NB_SCENE_HOST_ONLY");
   if (pt->globals.bounces + 2 > kMaxBounceSlots) return fail(NB_ERR_INVALID_ARG, "bounces too large");
   cudaStream_t st = (cudaStream_t)stream;
-  NB_CUDA(cudaMemsetAsync(pt->d_status, 0, sizeof(uint32_t), st), "cudaMemsetAsync");
-  NB_CUDA(cudaMemsetAsync(pt->d_rays, 0, sizeof(unsigned long long), st), "cudaMemsetAsync");
+  // the status word and, behind it, the ray count
+  NB_CUDA(cudaMemsetAsync(pt->d_status, 0, (size_t)((char*)(pt->d_rays + 1) - (char*)pt->d_status), st),
+          "cudaMemsetAsync");
   if (pt->globals.sample >= pt->max_sample_count) return fail(NB_ERR_EXHAUSTED, "sample count exhausted");
   const uint32_t npix = pt->width * pt->height;
   if (npix == 0 || n_samples == 0) return NB_OK;
@@ -664,22 +665,20 @@ static int render_samples(nb_pathtracer* pt, const nb_scene* scene, const nb_cam
     const uint32_t B = pt->globals.bounces;
     const bool nee = (pt->sampling & NB_SAMPLE_ENV_NEE) != 0 && !pt->cache;
     jp.flags = nee ? kJobEnvNee : 0u;
-    wt.flags = (nee || pt->cache) ? kWaveZeroRadiance : 0u;  // their shading adds to radiance
-    if (nee) {
-      if ((rc = ensure_shadow(pt, npix * S))) return rc;
-      NB_CUDA(cudaMemsetAsync(pt->sq.counts, 0, 2 * kMaxBounceSlots * sizeof(uint32_t), st), "cudaMemsetAsync");
-    }
+    if (nee && (rc = ensure_shadow(pt, npix * S))) return rc;
     CacheWave cw{};
     if (pt->cache) {
       rc = cache_wave_begin(pt->cache, scene, wt.n_paths, &cw, st);
       if (rc) return rc;
     }
-    cudaError_t e = timed_launch(pt, kKindRaygen, st, [&] { return launch_raygen(pb, wt, pt->sms, st); });
-    if (e == cudaSuccess)
-      e = launch_bounces(pb, wt, pt->cache ? Estimator::kCache : nee ? Estimator::kNee : Estimator::kPlain, true, B,
-                         pt->sq, cw, pt->d_rays, pt->sms, st, true, pt->d_trace_counts, [&](bool trace, auto launch) {
-                           return timed_launch(pt, trace ? kKindTrace : kKindShade, st, launch);
-                         });
+    cudaError_t e = launch_bounces(pb, wt, pt->cache ? Estimator::kCache : nee ? Estimator::kNee : Estimator::kPlain,
+                                   true, B, pt->sq, cw, pt->d_rays, pt->sms, st, true, pt->d_trace_counts,
+                                   [&](Stage stage, auto launch) {
+                                     const int kind = stage == Stage::kStart   ? kKindRaygen
+                                                      : stage == Stage::kTrace ? kKindTrace
+                                                                               : kKindShade;
+                                     return timed_launch(pt, kind, st, launch);
+                                   });
     if (e == cudaSuccess && pt->cache) {
       rc = NB_OK;
       e = timed_launch(pt, kKindCacheInfer, st, [&] {
@@ -880,14 +879,19 @@ int nb_pathtracer_last_stats(const nb_pathtracer* pt, uint64_t* rays, uint32_t* 
 }
 
 // ---- traversal queries -------------------------------------------------------------------
-static int check_status(const nb_scene* scene, cudaStream_t st, uint32_t* out = nullptr) {
-  uint32_t s = 0;
-  NB_CUDA(cudaMemcpyAsync(&s, scene->d_status, sizeof(s), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
-  NB_CUDA(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-  if (out) *out = s;
+static int status_code(uint32_t s) {
   if (s & nbd::kStatusStackOverflow) return fail(NB_ERR_STACK_OVERFLOW, "traversal stack overflow");
   if (s & nbd::kStatusIterationCap) return fail(NB_ERR_TIMEOUT, "traversal iteration cap reached");
   return NB_OK;
+}
+static int check_status(const nb_scene* scene, cudaStream_t st, uint32_t* out = nullptr) {
+  uint32_t s = 0;
+  const int64_t host = scene->host_query.status.load();
+  if (host >= 0) s = (uint32_t)host;
+  else NB_CUDA(cudaMemcpyAsync(&s, scene->d_status, sizeof(s), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+  NB_CUDA(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+  if (out) *out = s;
+  return status_code(s);
 }
 
 int nb_scene_status(const nb_scene* scene, uint32_t* status, void* stream) {
@@ -903,6 +907,7 @@ int nb_trace_rays(const nb_scene* scene, const float* rays, size_t n, uint32_t f
   if (n > 0xFFFFFFE0ull) return fail(NB_ERR_INVALID_ARG, "too many rays in one call");
   if (!scene->uploaded) return fail(NB_ERR_INVALID_ARG, "scene was built with NB_SCENE_HOST_ONLY");
   cudaStream_t st = (cudaStream_t)stream;
+  scene->host_query.status.store(-1);
   NB_CUDA(cudaMemsetAsync(scene->d_status, 0, sizeof(uint32_t), st), "cudaMemsetAsync");
   cudaError_t e = launch_trace_rays(scene->dev, rays, (uint32_t)n, (flags & NB_TRACE_ANY) != 0,
                                     (flags & NB_TRACE_INCOHERENT) != 0, hits, instances,
@@ -911,12 +916,51 @@ int nb_trace_rays(const nb_scene* scene, const float* rays, size_t n, uint32_t f
   return NB_OK;
 }
 
+// nb_trace_rays_host through the scene's page-locked buffer (1 <= n <= kGroupPaths)
+static int trace_rays_pinned(const nb_scene* scene, const float* rays, size_t n, uint32_t flags, float* hits,
+                             uint32_t* instances, cudaStream_t st) {
+  HostQuery& q = scene->host_query;
+  std::lock_guard<std::mutex> lk(q.mu);
+  const size_t need = 64 + n * (32 + 16 + 4);
+  if (q.bytes < need) {
+    if (q.mem) cudaFreeHost(q.mem);
+    q.mem = nullptr;
+    q.bytes = 0;
+    size_t bytes = 1 << 16;
+    while (bytes < need) bytes *= 2;
+    void* p = nullptr;
+    NB_CUDA(cudaHostAlloc(&p, bytes, cudaHostAllocPortable), "cudaHostAlloc(host query)");
+    q.mem = (char*)p;
+    q.bytes = bytes;
+  }
+  uint32_t* status = (uint32_t*)q.mem;
+  float* r = (float*)(q.mem + 64);
+  float* h = r + 8 * n;
+  uint32_t* inst = (uint32_t*)(h + 4 * n);
+  *status = 0;
+  std::memcpy(r, rays, n * 32);
+  cudaError_t e = launch_trace_rays(scene->dev, r, (uint32_t)n, (flags & NB_TRACE_ANY) != 0,
+                                    (flags & NB_TRACE_INCOHERENT) != 0, h, instances ? inst : nullptr, scene->d_fetch,
+                                    status, scene->sms, st);
+  const cudaError_t done = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = done;
+  if (e != cudaSuccess) return cuda_fail(e, "trace launch");
+  std::memcpy(hits, h, n * 16);
+  if (instances) std::memcpy(instances, inst, n * 4);
+  const uint32_t bits = *(volatile uint32_t*)status;
+  q.status.store(bits);
+  return status_code(bits);
+}
+
 int nb_trace_rays_host(const nb_scene* scene, const float* rays, size_t n, uint32_t flags, float* hits,
                        uint32_t* instances, void* stream) {
   if (!scene || (n && (!rays || !hits))) return fail(NB_ERR_INVALID_ARG, "NULL argument");
   if (n > 0xFFFFFFE0ull) return fail(NB_ERR_INVALID_ARG, "too many rays in one call");
   if (!scene->uploaded) return fail(NB_ERR_INVALID_ARG, "scene was built with NB_SCENE_HOST_ONLY");
   cudaStream_t st = (cudaStream_t)stream;
+  if (flags & ~(uint32_t)(NB_TRACE_ANY | NB_TRACE_INCOHERENT))
+    return fail(NB_ERR_INVALID_ARG, "unknown trace flags 0x%x", flags);
+  if (n >= 1 && n <= kGroupPaths) return trace_rays_pinned(scene, rays, n, flags, hits, instances, st);
   DeviceArena tmp;
   void *dr = nullptr, *dh = nullptr, *di = nullptr;
   int rc;

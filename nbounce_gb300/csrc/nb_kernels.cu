@@ -681,11 +681,15 @@ __device__ __forceinline__ uint32_t first_group_item() {
   return (lane / kGroupLanes * (kGroupThreads / 32) + warp) * gridDim.x + blockIdx.x;
 }
 // The next one of a group that wants one: *fetch counts the items taken beyond the first of every
-// group.  All lanes of the warp call it.
-__device__ __forceinline__ void next_group_item(const Group& g, uint32_t* fetch, bool want, uint32_t& i) {
-  uint32_t r = 0;
-  if (want && g.sub == 0) r = gridDim.x * kGroupsPerBlock + atomicAdd(fetch, 1u);
-  r = g.shfl(r, 0);
+// group; with at most one item per group there is none, and the cursor is not touched.  All lanes of
+// the warp call it.
+__device__ __forceinline__ void next_group_item(const Group& g, uint32_t* fetch, uint32_t n, bool want, uint32_t& i) {
+  const uint32_t groups = gridDim.x * kGroupsPerBlock;
+  uint32_t r = n;
+  if (n > groups) {
+    if (want && g.sub == 0) r = groups + atomicAdd(fetch, 1u);
+    r = g.shfl(r, 0);
+  }
   if (want) i = r;
 }
 
@@ -712,7 +716,7 @@ __global__ void __launch_bounds__(kGroupThreads, 6)
         hits[i] = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.tri));
         if (inst) inst[i] = t.h.inst;
       }
-      next_group_item(g, fetch, done, i);
+      next_group_item(g, fetch, n, done, i);
       fresh = fresh || done;
     }
   }
@@ -1864,6 +1868,27 @@ __global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(P
   if (st) atomicOr(pb.status, st);
 }
 
+__device__ __forceinline__ void accumulate_sample(float4& c, V3 L, uint32_t sample) {
+  const float w = 1.0f / (float)sample;
+  c.x = c.x * (1.0f - w) + L.x * w;
+  c.y = c.y * (1.0f - w) + L.y * w;
+  c.z = c.z * (1.0f - w) + L.z * w;
+}
+// A path's final radiance: kept for k_accumulate, or (kWaveDirect) added to its pixel.
+__device__ __forceinline__ void put_radiance(const PathBatch& pb, const WaveTables& wt, const Segment* segs,
+                                             uint32_t id, V3 L, bool lead) {
+  if (!lead) return;
+  if (!(wt.flags & nb::kWaveDirect)) {
+    pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f);
+    return;
+  }
+  const Segment sg = segs[find_segment<false>(segs, wt.n_segs, id)];
+  float4* out = wt.jobs[sg.job].out + (id - sg.path_begin);
+  float4 c = *out;
+  accumulate_sample(c, L, sg.first_sample);
+  *out = make_float4(c.x, c.y, c.z, 1.0f);
+}
+
 // Paths run to their ends, 8 lanes per path (GroupTrace): the camera paths of a small wave
 // (bounce0 = 0), or the queue of a bounce that no longer fills the GPU (queue_count).  Traversal and
 // shading of a path follow one another here without a launch between them, so the time is that of
@@ -1871,6 +1896,8 @@ __global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(P
 // group shade the same vertex; lane 0 writes.  Samples, arithmetic and the order of a path's
 // radiance additions are those of the per-bounce kernels.  Bound by the latency of a path's steps
 // (0.8 us each) and, from ~16K paths on, by instruction issue (54%).
+// With kWaveDirect (one sample per pixel, reference or NEE estimator) a path adds its radiance to its
+// pixel itself (accumulate_sample) and the wave needs no other launch.
 enum EstimatorKind : int { kEstPlain, kEstNee, kEstCache };
 template <int kEst>
 __global__ void __launch_bounds__(kGroupThreads, 4)
@@ -1901,6 +1928,7 @@ __global__ void __launch_bounds__(kGroupThreads, 4)
         camera_ray(segs, wt, pb, i, ray.o, ray.d);
         ray.t = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
         acc = zero;
+        if (kEst == kEstCache && lead) pb.radiance[__float_as_uint(ray.o.w)] = zero;  // lookups add to it
       } else {
         ray.o = (odd ? pb.q_o[1] : pb.q_o[0])[i];
         ray.d = (odd ? pb.q_d[1] : pb.q_d[0])[i];
@@ -1927,9 +1955,7 @@ __global__ void __launch_bounds__(kGroupThreads, 4)
         const float4 H = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.tri));
         const float4 O = ray.o, D = ray.d, T = ray.t;
         const auto inst = [&] { return t.h.inst; };
-        const auto end = [&](uint32_t id, V3 L) {
-          if (lead) pb.radiance[id] = make_float4(L.x, L.y, L.z, 0.0f);
-        };
+        const auto end = [&](uint32_t id, V3 L) { put_radiance(pb, wt, segs, id, L, lead); };
         if (kEst == kEstPlain) {
           cont = shade_plain(pb, wt, segs, b, O, D, H, T, inst, end, ray);
         } else if (kEst == kEstNee) {
@@ -1969,12 +1995,12 @@ __global__ void __launch_bounds__(kGroupThreads, 4)
         ++rays;
         t.begin(wt.scenes[scene], xyz(ray.o), xyz(ray.d), false);
       } else {
-        if (kEst == kEstNee && lead) pb.radiance[__float_as_uint(ray.o.w)] = acc;
+        if (kEst == kEstNee) put_radiance(pb, wt, segs, __float_as_uint(ray.o.w), xyz(acc), lead);
         ended = true;
       }
     traced:;
     }
-    next_group_item(g, pb.fetch + bounce0, ended, i);
+    next_group_item(g, pb.fetch + bounce0, n, ended, i);
     fresh = ended;
   }
   if (lead) {
@@ -2000,13 +2026,8 @@ __global__ void __launch_bounds__(256) k_accumulate(PathBatch pb, const WaveTabl
     const JobParams& jp = wt.jobs[sg.job];
     const uint32_t pix = t - sg.pix_begin;
     float4 c = jp.out[pix];
-    for (uint32_t k = 0; k < sg.n_samples; ++k) {
-      const float w = 1.0f / (float)(sg.first_sample + k);
-      const float4 L = pb.radiance[(size_t)sg.path_begin + (size_t)k * jp.npix + pix];
-      c.x = c.x * (1.0f - w) + L.x * w;
-      c.y = c.y * (1.0f - w) + L.y * w;
-      c.z = c.z * (1.0f - w) + L.z * w;
-    }
+    for (uint32_t k = 0; k < sg.n_samples; ++k)
+      accumulate_sample(c, xyz(pb.radiance[(size_t)sg.path_begin + (size_t)k * jp.npix + pix]), sg.first_sample + k);
     jp.out[pix] = make_float4(c.x, c.y, c.z, 1.0f);
   }
 }
@@ -2028,18 +2049,23 @@ static int blocks_for(const void* kernel, int threads, int sms) {
 cudaError_t launch_trace_rays(const nbd::DevScene& s, const float* rays, uint32_t n, bool any, bool refill,
                               float* hits, uint32_t* inst, uint32_t* fetch, uint32_t* status, int sms,
                               cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
   if (n <= kGroupPaths) {
     const void* kernel = any ? (const void*)nbd::k_trace_rays_group<true> : (const void*)nbd::k_trace_rays_group<false>;
     static const int full[2] = {blocks_for((const void*)nbd::k_trace_rays_group<false>, nbd::kGroupThreads, sms),
                                 blocks_for((const void*)nbd::k_trace_rays_group<true>, nbd::kGroupThreads, sms)};
+    const unsigned blocks = (unsigned)std::min(full[any], (int)n);
+    if (n > blocks * nbd::kGroupsPerBlock) {
+      const cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st);
+      if (e != cudaSuccess) return e;
+    }
     const float4* r4 = (const float4*)rays;
     float4* h4 = (float4*)hits;
     void* args[] = {(void*)&s, (void*)&r4, (void*)&n, (void*)&h4, (void*)&inst, (void*)&fetch, (void*)&status};
-    return cudaLaunchKernel(kernel, dim3((unsigned)std::min(full[any], (int)n)), dim3(nbd::kGroupThreads), args, 0, st);
+    return cudaLaunchKernel(kernel, dim3(blocks), dim3(nbd::kGroupThreads), args, 0, st);
   }
+  const cudaError_t e = cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st);
+  if (e != cudaSuccess) return e;
 #define NB_TRACE_RAYS(A, R)                                                                            \
   {                                                                                                    \
     static const int g = blocks_for((const void*)nbd::k_trace_rays<A, R>, nbd::kTraceThreads, sms);                  \
@@ -2113,11 +2139,15 @@ cudaError_t launch_trace_shadow(const PathBatch& pb, const WaveTables& wt, const
 
 cudaError_t launch_trace_paths(const PathBatch& pb, const WaveTables& wt, Estimator est, const CacheWave& cw,
                                uint32_t bounce, unsigned long long* ray_total, int sms, cudaStream_t st) {
-#define NB_TRACE_PATHS(E)                                                                                  \
-  {                                                                                                        \
-    static const int g = blocks_for((const void*)nbd::k_trace_paths<E>, nbd::kGroupThreads, sms);          \
-    const int blocks = (int)std::min<uint64_t>((uint64_t)g, wt.n_paths);                                   \
-    nbd::k_trace_paths<E><<<blocks, nbd::kGroupThreads, 0, st>>>(pb, wt, cw, bounce, ray_total);           \
+#define NB_TRACE_PATHS(E)                                                                                   \
+  {                                                                                                         \
+    static const int g = blocks_for((const void*)nbd::k_trace_paths<E>, nbd::kGroupThreads, sms);           \
+    const unsigned blocks = (unsigned)std::min<uint64_t>((uint64_t)g, wt.n_paths);                          \
+    if (bounce == 0 && wt.n_paths > blocks * nbd::kGroupsPerBlock) { /* a whole wave: no k_raygen before */ \
+      const cudaError_t e = cudaMemsetAsync(pb.fetch, 0, sizeof(uint32_t), st);                             \
+      if (e != cudaSuccess) return e;                                                                       \
+    }                                                                                                       \
+    nbd::k_trace_paths<E><<<blocks, nbd::kGroupThreads, 0, st>>>(pb, wt, cw, bounce, ray_total);            \
   }
   if (est == Estimator::kPlain) NB_TRACE_PATHS(nbd::kEstPlain)
   else if (est == Estimator::kNee) NB_TRACE_PATHS(nbd::kEstNee)
@@ -2135,6 +2165,7 @@ cudaError_t launch_env_sample(const nbd::DevEnv& env, const float* u, uint32_t n
 }
 
 cudaError_t launch_accumulate(const PathBatch& pb, const WaveTables& wt, int sms, cudaStream_t st) {
+  if (wt.flags & kWaveDirect) return cudaSuccess;
   int g = (int)std::min<uint64_t>((wt.n_pix + 255) / 256, (uint64_t)sms * 16);
   nbd::k_accumulate<<<g < 1 ? 1 : g, 256, 0, st>>>(pb, wt);
   return cudaGetLastError();

@@ -44,7 +44,9 @@ struct Segment {
 // flags: kWaveZeroRadiance - raygen zeroes every path's radiance, for waves whose shading adds
 // to it (environment NEE, radiance cache); with the reference estimator every path's radiance
 // is written once, where the path ends (k_shade), and raygen leaves it alone.
+// kWaveDirect - the wave is one launch of k_trace_paths whose paths add to their pixels themselves.
 constexpr uint32_t kWaveZeroRadiance = 1u << 0;
+constexpr uint32_t kWaveDirect = 1u << 1;
 // 64-bit counters per bounce slot of the instrumented traversal (nb_pathtracer_trace_counters):
 // 0-4 node / triangle / instance / push counts, 5 rays, 6-10 warp-step statistics
 constexpr uint32_t kTraceCounterSlots = 16;
@@ -109,6 +111,7 @@ struct CacheWave;
 // radiance-cache mode shade (nb_mlp.cuh describes the wave state)
 cudaError_t launch_shade_cache(const PathBatch& pb, const WaveTables& wt, const CacheWave& cw, uint32_t bounce,
                                int sms, cudaStream_t st);
+// nothing to do for a kWaveDirect wave
 cudaError_t launch_accumulate(const PathBatch& pb, const WaveTables& wt, int sms, cudaStream_t st);
 
 enum class Estimator { kPlain, kNee, kCache };
@@ -126,38 +129,53 @@ cudaError_t launch_trace_paths(const PathBatch& pb, const WaveTables& wt, Estima
 // launches alone), 256x256 at 16 spp 608 / 580 / 570 / 600 us (720), 64x48 at 1 spp 69 us (339).
 constexpr uint32_t kGroupPaths = 1u << 16;
 
-// All bounces of a wave.  groups: short queues go to k_trace_paths.  counters (optional): the
-// instrumented traversal, a ray per lane throughout.  timed(trace, launch) runs one launch (trace:
-// traversal, else shading).
+// The launch kinds of a wave (nb_kernel_times)
+enum class Stage { kStart, kTrace, kShade };
+
+// A wave from its start to its last bounce.  groups: short queues go to k_trace_paths.  counters
+// (optional): the instrumented traversal, a ray per lane throughout.  timed(stage, launch) runs one
+// launch.  launch_accumulate has to follow (after the lookups of a cache wave).
 template <class Timed>
 cudaError_t launch_bounces(const PathBatch& pb, WaveTables& wt, Estimator est, bool single_scene, uint32_t max_bounces,
                            const ShadowQueue& sq, const CacheWave& cw, unsigned long long* ray_total, int sms,
                            cudaStream_t st, bool groups, unsigned long long* counters, Timed timed) {
   groups = groups && counters == nullptr;
   wt.group_limit = groups ? kGroupPaths : 0u;
+  wt.flags = est != Estimator::kPlain ? kWaveZeroRadiance : 0u;  // their shading adds to radiance
   // From bounce `last` on every queue goes to k_trace_paths, whatever its length, and the launches of
   // later bounces are saved: there the queue holds at most kGroupPaths paths if half of the paths end
   // per bounce (half to two thirds do in open scenes; where most survive, both ways took the same time
   // within 10%).
   uint32_t last = 0;
   while (groups && (wt.n_paths >> last) > kGroupPaths) ++last;
+  auto paths = [&](uint32_t b) {
+    wt.group_limit = b == last ? 0xFFFFFFFFu : kGroupPaths;
+    return timed(Stage::kTrace, [&] { return launch_trace_paths(pb, wt, est, cw, b, ray_total, sms, st); });
+  };
+  if (groups && last == 0) {
+    bool direct = est != Estimator::kCache;
+    for (uint32_t k = 0; k < wt.n_segs; ++k) direct = direct && wt.segs[k].n_samples == 1;
+    wt.flags = direct ? kWaveDirect : 0u;
+    return paths(0);
+  }
   cudaError_t e = cudaSuccess;
+  if (est == Estimator::kNee) e = cudaMemsetAsync(sq.counts, 0, 2 * kMaxBounceSlots * sizeof(uint32_t), st);
+  if (e == cudaSuccess) e = timed(Stage::kStart, [&] { return launch_raygen(pb, wt, sms, st); });
   for (uint32_t b = 0; b <= max_bounces && e == cudaSuccess; ++b) {
-    if (groups && (b >= 1 || last == 0)) {
-      wt.group_limit = b == last ? 0xFFFFFFFFu : kGroupPaths;
-      e = timed(true, [&] { return launch_trace_paths(pb, wt, est, cw, b, ray_total, sms, st); });
+    if (groups && b >= 1) {
+      e = paths(b);
       if (b == last) return e;
     }
     if (e == cudaSuccess)
-      e = timed(true, [&] { return launch_trace_wave(pb, wt, single_scene, b, ray_total, sms, st, counters); });
+      e = timed(Stage::kTrace, [&] { return launch_trace_wave(pb, wt, single_scene, b, ray_total, sms, st, counters); });
     if (e == cudaSuccess)
-      e = timed(false, [&] {
+      e = timed(Stage::kShade, [&] {
         return est == Estimator::kCache ? launch_shade_cache(pb, wt, cw, b, sms, st)
                : est == Estimator::kNee ? launch_shade_nee(pb, wt, sq, b, sms, st)
                                         : launch_shade(pb, wt, b, sms, st);
       });
     if (e == cudaSuccess && est == Estimator::kNee)
-      e = timed(true, [&] { return launch_trace_shadow(pb, wt, sq, b, sms, st); });
+      e = timed(Stage::kTrace, [&] { return launch_trace_shadow(pb, wt, sq, b, sms, st); });
   }
   return e;
 }

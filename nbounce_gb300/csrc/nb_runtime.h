@@ -2,7 +2,9 @@
 // CUDA error mapping, the device allocation arena and the scene / environment handles.
 #pragma once
 
+#include <atomic>
 #include <cstdio>
+#include <mutex>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -79,6 +81,20 @@ int parse_dds_cube(const uint8_t* bytes, size_t n, DdsCube* out);
 
 }  // namespace nb
 
+// Page-locked buffer of nb_trace_rays_host: short queries read their rays from it and write their hits
+// into it, so that a call needs no device allocations and no copy commands.  Kept with the scene, at
+// most kGroupPaths rays' worth (3.4 MB); calls on the same scene take turns.
+struct HostQuery {
+  std::mutex mu;
+  char* mem = nullptr;
+  size_t bytes = 0;
+  // status bits of the last query if it ran through this buffer, else -1 (d_status has them)
+  std::atomic<int64_t> status{-1};
+  ~HostQuery() {
+    if (mem) cudaFreeHost(mem);
+  }
+};
+
 struct nb_scene {
   nb::HostScene host;
   nbd::DevScene dev{};
@@ -87,6 +103,7 @@ struct nb_scene {
   uint32_t* d_status = nullptr;
   int sms = 1;
   bool uploaded = false;
+  mutable HostQuery host_query;
 };
 
 struct nb_env {

@@ -323,20 +323,17 @@ struct nb_server {
     return false;
   }
 
-  // A small wave stays on the per-bounce kernels: with 8 lanes per path the server drains small jobs
-  // about as fast as a caller can submit them, and a queue limit would then not shed any (a burst of
-  // 200 jobs of 64x64 pixels at 16,384 paths per wave).
-  bool group_wave() const { return wt->n_paths > 4 * kGroupPaths; }
+  // A wave of at most kServerPerBounce paths stays on the per-bounce kernels: with 8 lanes per path the
+  // server drains tiny jobs about as fast as a caller can submit them, and a queue limit would then not
+  // shed any (a burst of 200 jobs of 64x64 pixels at 16,384 paths per wave).
+  static constexpr uint32_t kServerPerBounce = 1u << 14;
+  bool group_wave() const { return wt->n_paths > kServerPerBounce; }
 
   cudaError_t launch_wave(uint32_t max_bounces, bool single_scene, bool nee) {
     PathBatch p = pb;
-    cudaError_t e = cudaSuccess;
-    wt->flags = nee ? kWaveZeroRadiance : 0u;  // NEE shading adds to radiance
-    if (nee) e = cudaMemsetAsync(sq.counts, 0, 2 * kMaxBounceSlots * sizeof(uint32_t), stream);
-    if (e == cudaSuccess) e = launch_raygen(p, *wt, sms, stream);
-    if (e == cudaSuccess)
-      e = launch_bounces(p, *wt, nee ? Estimator::kNee : Estimator::kPlain, single_scene, max_bounces, sq, CacheWave{},
-                         d_rays, sms, stream, group_wave(), nullptr, [](bool, auto launch) { return launch(); });
+    cudaError_t e = launch_bounces(p, *wt, nee ? Estimator::kNee : Estimator::kPlain, single_scene, max_bounces, sq,
+                                   CacheWave{}, d_rays, sms, stream, group_wave(), nullptr,
+                                   [](Stage, auto launch) { return launch(); });
     if (e == cudaSuccess) e = launch_accumulate(p, *wt, sms, stream);
     return e;
   }
@@ -358,11 +355,8 @@ struct nb_server {
   int launch_cache_wave(nb_cache* c, const CacheWave& cw, uint32_t max_bounces) {
     int rc = NB_OK;
     PathBatch p = pb;
-    wt->flags = kWaveZeroRadiance;  // cache lookups add to radiance
-    cudaError_t e = launch_raygen(p, *wt, sms, stream);
-    if (e == cudaSuccess)
-      e = launch_bounces(p, *wt, Estimator::kCache, true, max_bounces, sq, cw, d_rays, sms, stream, group_wave(), nullptr,
-                         [](bool, auto launch) { return launch(); });
+    cudaError_t e = launch_bounces(p, *wt, Estimator::kCache, true, max_bounces, sq, cw, d_rays, sms, stream,
+                                   group_wave(), nullptr, [](Stage, auto launch) { return launch(); });
     if (e != cudaSuccess) return cuda_fail(e, "cache wave launch");
     if ((rc = cache_wave_infer(c, p, sms, stream)) || (rc = cache_wave_train(c, wt->n_paths, sms, stream)))
       return rc;

@@ -122,7 +122,6 @@ extern "C" int nb_render_static(const nb_scene* scene, const nb_env* env, const 
 
   WaveTables& wt = g_tables;
   wt.n_jobs = wt.n_scenes = wt.n_segs = 1;
-  wt.flags = 0u;  // reference estimator: every path's radiance is written where it ends
   wt.scenes[0] = scene->dev;
   JobParams& jp = wt.jobs[0];
   std::memcpy(jp.c2w, camera->clip_to_world, sizeof(jp.c2w));
@@ -141,10 +140,8 @@ extern "C" int nb_render_static(const nb_scene* scene, const nb_env* env, const 
     wt.segs[0] = Segment{0u, first_sample + done, S, 0u, 0u};
     wt.n_paths = (uint32_t)npix * S;
     wt.n_pix = (uint32_t)npix;
-    e = launch_raygen(pb, wt, sms, st);
-    if (e == cudaSuccess)
-      e = launch_bounces(pb, wt, Estimator::kPlain, true, bounces, ShadowQueue{}, CacheWave{}, rays, sms, st, true, nullptr,
-                         [](bool, auto launch) { return launch(); });
+    e = launch_bounces(pb, wt, Estimator::kPlain, true, bounces, ShadowQueue{}, CacheWave{}, rays, sms, st, true, nullptr,
+                       [](Stage, auto launch) { return launch(); });
     if (e == cudaSuccess) e = launch_accumulate(pb, wt, sms, st);
     done += S;
   }

@@ -99,3 +99,42 @@ def test_cache_frames_equal_ray_per_lane(world, w, h, spread):
         out.append((pt.download(), cache.get_weights(), pt.last_stats(), stats["queries"], stats["records_found"]))
     for x, y in zip(*out):
         assert np.array_equal(np.asarray(x), np.asarray(y), equal_nan=True)
+
+
+def test_host_and_device_queries_alternate(world):
+    """Host queries of changing sizes (through the scene's own buffer up to 65,536 rays, through device
+    buffers beyond) and device queries on the same scene give the same hits; nb_scene_status follows the
+    last query; calls from several threads take turns."""
+    import threading
+
+    import torch
+    scene = world["instanced"][0]
+    n = LIMIT + 5
+    rays = scenes.incoherent_rays(n, seed=21)
+    rays[:, :3] *= np.float32([30.0, 12.0, 30.0])
+    dev = torch.from_numpy(rays).cuda()
+    hits = torch.empty(n, 4, device="cuda")
+    inst = torch.empty(n, dtype=torch.int32, device="cuda")
+    scene.trace_device(dev.data_ptr(), n, hits.data_ptr(), inst.data_ptr(), incoherent=True)
+    assert scene.status() == 0
+    want, want_i = hits.cpu().numpy().view(np.uint32), inst.cpu().numpy().view(np.uint32)
+    for m in (1, 700, 30000, 5, n, 1, LIMIT):
+        h, i = scene.trace_host(rays[:m], incoherent=True)
+        assert np.array_equal(h.view(np.uint32), want[:m]) and np.array_equal(i, want_i[:m])
+        h, none = scene.trace_host(rays[:m], with_instances=False)
+        assert none is None and np.array_equal(h.view(np.uint32), want[:m]) and scene.status() == 0
+    assert scene.trace_host(rays[:0])[0].shape == (0, 4)
+    bad = []
+
+    def query(lo):
+        for _ in range(20):
+            h, _ = scene.trace_host(rays[lo:lo + 900])
+            if not np.array_equal(h.view(np.uint32), want[lo:lo + 900]):
+                bad.append(lo)
+
+    threads = [threading.Thread(target=query, args=(1000 * k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
