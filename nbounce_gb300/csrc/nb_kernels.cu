@@ -580,9 +580,12 @@ __device__ __forceinline__ uint32_t trace_ray(const DevScene& s, const V3 wo, co
 // refill most lanes would idle while the longest ray of each 32 finishes.  Refill changes only
 // which lane traces a ray, not its result.
 constexpr uint32_t kRefillIdle = 6;
-template <bool kAny, bool kCount, class Load, class SceneOf, class Finish>
+// kMixed: rays from any_from on are any-hit queries among closest-hit ones; such a ray ends with the node
+// step that finds its hit.
+template <bool kAny, bool kCount, bool kMixed = false, class Load, class SceneOf, class Finish>
 __device__ __forceinline__ uint32_t trace_refill(uint32_t* fetch, uint32_t n, Load load, SceneOf scene, Finish finish,
-                                                 TraceCount* cnt, float* world, uint2* entries) {
+                                                 TraceCount* cnt, float* world, uint2* entries,
+                                                 uint32_t any_from = 0xFFFFFFFFu) {
   const WorldShared wr{world};
   const uint32_t lane = threadIdx.x & 31u;
   TraceState t;
@@ -610,7 +613,8 @@ __device__ __forceinline__ uint32_t trace_refill(uint32_t* fetch, uint32_t n, Lo
         }
       }
     }
-    if (my != kNone && !trace_step<kAny, kCount>(t, SharedStack{stack, entries}, scene(sidx), cnt, wr)) {
+    if (my != kNone && (!trace_step<kAny, kCount>(t, SharedStack{stack, entries}, scene(sidx), cnt, wr) ||
+                        (kMixed && my >= any_from && t.t_hit < kNoHit))) {
       finish(my, t.t_hit, stack[kHitSlot], stack[kHitSlot + 1]);
       st |= t.status;
       my = kNone;
@@ -851,6 +855,14 @@ __device__ __forceinline__ uint32_t queue_count(const PathBatch& pb, const WaveT
   return n <= wt.group_limit ? 0u : n;
 }
 
+// An unoccluded shadow ray adds its contribution to the path.  A path has at most one shadow ray per
+// bounce, so each radiance entry has one writer per launch.
+__device__ __forceinline__ void add_shadow(const PathBatch& pb, const ShadowQueue& sq, uint32_t r) {
+  const uint32_t id = __float_as_uint(sq.o[r].w);
+  const float4 c = sq.c[r], rr = pb.radiance[id];
+  pb.radiance[id] = make_float4(rr.x + c.x, rr.y + c.y, rr.z + c.z, 0.0f);
+}
+
 // kSingle: every ray of the wave uses wt.scenes[0]; else the scene index carried in q_d.w.
 // Bounce 0 (camera rays): persistent warps take 32 consecutive queue entries per atomic - 32
 // samples of one pixel - make each lane's camera ray (camera_ray), write it to the queue for
@@ -868,13 +880,18 @@ __device__ __forceinline__ uint32_t queue_count(const PathBatch& pb, const WaveT
 // lanes active per instruction on bounce 1).  Camera rays keep whole-warp chunks: a warp's 32
 // samples of one pixel finish together, and refilling them measured 9% slower traversal.
 // Refill changes only which lane traces a ray, not its result.
-template <bool kSingle, bool kCount, bool kRefill>
+// kShadow (lane refill only): the launch also traces the shadow rays that the bounce before queued
+// (environment NEE), after the queue's rays.  They are independent of this bounce's rays, and in a
+// launch of their own they added the tail of their longest ray to every bounce (~100 us of a
+// 1-2 M path wave): 1013x571 at 3 spp with NEE 4.04 -> 3.66 ms.
+template <bool kSingle, bool kCount, bool kRefill, bool kShadow = false>
 __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChunkBlocks) k_trace_wave(PathBatch pb, const WaveTables wt,
                                                                      uint32_t bounce,
                                                        unsigned long long* __restrict__ ray_total,
-                                                       unsigned long long* __restrict__ counters) {
-  const uint32_t n = queue_count(pb, wt, bounce);
-  if (n == 0) return;
+                                                       unsigned long long* __restrict__ counters,
+                                                       const ShadowQueue sq) {
+  const uint32_t n = queue_count(pb, wt, bounce), n_shadow = kShadow ? sq.counts[bounce - 1u] : 0u;
+  if (n + n_shadow == 0) return;
   __shared__ DevScene scenes[kSingle ? 1 : nb::kMaxWaveScenes];
   if (!kSingle) {
     for (uint32_t i = threadIdx.x; i < wt.n_scenes; i += blockDim.x) scenes[i] = wt.scenes[i];
@@ -918,20 +935,26 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChun
     __shared__ float world[kTraceWarps][kWorldFloats];
     __shared__ uint2 entries[kSharedEntries][kTraceThreads];
     const DevScene* sc = kSingle ? wt.scenes : scenes;
-    st = trace_refill<false, kCount>(
-        pb.fetch + bounce, n,
+    // (k_trace_paths takes the bounce's own cursor if the queue is short)
+    st = trace_refill<false, kCount, kShadow>(
+        kShadow ? sq.fetch + bounce - 1u : pb.fetch + bounce, n + n_shadow,
         [&](uint32_t r, V3& o, V3& d, uint32_t& sidx) {
-          const float4 o4 = qo[r], d4 = qd[r];
+          const bool shadow = kShadow && r >= n;
+          const float4 o4 = shadow ? sq.o[r - n] : qo[r], d4 = shadow ? sq.d[r - n] : qd[r];
           o = xyz(o4);
           d = xyz(d4);
           sidx = kSingle ? 0u : __float_as_uint(d4.w);
         },
         [&](uint32_t sidx) -> const DevScene& { return sc[sidx]; },
         [&](uint32_t r, float t_hit, uint2 uv, uint2 ti) {
+          if (kShadow && r >= n) {
+            if (t_hit == kNoHit) add_shadow(pb, sq, r - n);
+            return;
+          }
           pb.hits[r] = make_float4(t_hit, __uint_as_float(uv.x), __uint_as_float(uv.y), __uint_as_float(ti.x));
           pb.hit_inst[r] = ti.y;
         },
-        &cnt, world[threadIdx.x >> 5], &entries[0][threadIdx.x]);
+        &cnt, world[threadIdx.x >> 5], &entries[0][threadIdx.x], n);
   }
   if (st) atomicOr(pb.status, st);
   if (kCount) {  // counters[kTraceCounterSlots * bounce + 0..10]: see nb_pathtracer_trace_counters
@@ -946,7 +969,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChun
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(slot + 5, (unsigned long long)n);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(ray_total, (unsigned long long)n);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(ray_total, (unsigned long long)n);
 }
 
 // Cube-map face of a direction and its coordinates s, t in [-1, 1] on that face: the standard
@@ -1834,11 +1857,10 @@ __global__ void __launch_bounds__(kShadeExtThreads) k_shade_nee(PathBatch pb, co
   }
 }
 
-// Shadow rays of one bounce: an any-hit query each (raytracing_sw.wgsl's triangle test and
-// BIAS, so the ray leaves its own surface like the reference's extension rays), with lane
-// refill (trace_refill); unoccluded rays add their contribution to the path.  A path has at most one shadow ray per bounce, so
-// each radiance entry has one writer per launch.  .w of a shadow ray's direction is the index
-// of its scene in the wave.
+// Shadow rays of the last bounce (and, beside the instrumented traversal, of every bounce): an any-hit
+// query each (raytracing_sw.wgsl's triangle test and BIAS, so the ray leaves its own surface like the
+// reference's extension rays), with lane refill (trace_refill).  .w of a shadow ray's direction is the
+// index of its scene in the wave.
 __global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(PathBatch pb, const WaveTables wt, const ShadowQueue sq,
                                                       uint32_t bounce) {
   const uint32_t n = sq.counts[bounce];
@@ -1858,11 +1880,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(P
       },
       [&](uint32_t sidx) -> const DevScene& { return scenes[sidx]; },
       [&](uint32_t r, float t_hit, uint2, uint2) {
-        if (t_hit == kNoHit) {
-          const uint32_t id = __float_as_uint(sq.o[r].w);
-          const float4 c = sq.c[r], rr = pb.radiance[id];
-          pb.radiance[id] = make_float4(rr.x + c.x, rr.y + c.y, rr.z + c.z, 0.0f);
-        }
+        if (t_hit == kNoHit) add_shadow(pb, sq, r);
       },
       nullptr, world[threadIdx.x >> 5], &entries[0][threadIdx.x]);
   if (st) atomicOr(pb.status, st);
@@ -2087,13 +2105,14 @@ cudaError_t launch_raygen(const PathBatch& pb, const WaveTables& wt, int sms, cu
 }
 
 cudaError_t launch_trace_wave(const PathBatch& pb, const WaveTables& wt, bool single_scene, uint32_t bounce,
-                              unsigned long long* ray_total, int sms, cudaStream_t st,
+                              const ShadowQueue* shadow, unsigned long long* ray_total, int sms, cudaStream_t st,
                               unsigned long long* counters) {
   const bool refill = bounce >= 1;
-#define NB_TRACE_WAVE(S, C, R)                                                                \
-  {                                                                                           \
-    static const int g = blocks_for((const void*)nbd::k_trace_wave<S, C, R>, nbd::kTraceThreads, sms);       \
-    nbd::k_trace_wave<S, C, R><<<g, nbd::kTraceThreads, 0, st>>>(pb, wt, bounce, ray_total, counters);      \
+  const ShadowQueue sq = shadow ? *shadow : ShadowQueue{};
+#define NB_TRACE_WAVE(S, C, ...)                                                                              \
+  {                                                                                                           \
+    static const int g = blocks_for((const void*)nbd::k_trace_wave<S, C, __VA_ARGS__>, nbd::kTraceThreads, sms); \
+    nbd::k_trace_wave<S, C, __VA_ARGS__><<<g, nbd::kTraceThreads, 0, st>>>(pb, wt, bounce, ray_total, counters, sq); \
   }
   if (counters) {
     if (single_scene) {
@@ -2101,6 +2120,8 @@ cudaError_t launch_trace_wave(const PathBatch& pb, const WaveTables& wt, bool si
     } else {
       if (refill) NB_TRACE_WAVE(false, true, true) else NB_TRACE_WAVE(false, true, false)
     }
+  } else if (shadow && refill) {
+    if (single_scene) NB_TRACE_WAVE(true, false, true, true) else NB_TRACE_WAVE(false, false, true, true)
   } else if (single_scene) {
     if (refill) NB_TRACE_WAVE(true, false, true) else NB_TRACE_WAVE(true, false, false)
   } else {

@@ -81,12 +81,14 @@ cudaError_t launch_trace_rays(const nbd::DevScene& s, const float* rays, uint32_
                               cudaStream_t st);
 
 cudaError_t launch_raygen(const PathBatch& pb, const WaveTables& wt, int sms, cudaStream_t st);
+struct ShadowQueue;
 // single_scene: all paths use wt.scenes[0] (passed by value); otherwise each ray's scene index.
+// shadow (optional, bounce >= 1): also traces the shadow rays of the bounce before.
 // counters (optional): runs the instrumented traversal, which adds its work counters (TLAS
 // node tests, BLAS node tests, triangle tests, instance entries, stack pushes) to
 // counters[8 * bounce + 0..4].
 cudaError_t launch_trace_wave(const PathBatch& pb, const WaveTables& wt, bool single_scene, uint32_t bounce,
-                              unsigned long long* ray_total, int sms, cudaStream_t st,
+                              const ShadowQueue* shadow, unsigned long long* ray_total, int sms, cudaStream_t st,
                               unsigned long long* counters = nullptr);
 cudaError_t launch_shade(const PathBatch& pb, const WaveTables& wt, uint32_t bounce, int sms, cudaStream_t st);
 // Shadow rays of environment next-event estimation: one per path and bounce at most.
@@ -149,33 +151,39 @@ cudaError_t launch_bounces(const PathBatch& pb, WaveTables& wt, Estimator est, b
   uint32_t last = 0;
   while (groups && (wt.n_paths >> last) > kGroupPaths) ++last;
   auto paths = [&](uint32_t b) {
-    wt.group_limit = b == last ? 0xFFFFFFFFu : kGroupPaths;
     return timed(Stage::kTrace, [&] { return launch_trace_paths(pb, wt, est, cw, b, ray_total, sms, st); });
   };
   if (groups && last == 0) {
     bool direct = est != Estimator::kCache;
     for (uint32_t k = 0; k < wt.n_segs; ++k) direct = direct && wt.segs[k].n_samples == 1;
     wt.flags = direct ? kWaveDirect : 0u;
+    wt.group_limit = 0xFFFFFFFFu;
     return paths(0);
   }
   cudaError_t e = cudaSuccess;
   if (est == Estimator::kNee) e = cudaMemsetAsync(sq.counts, 0, 2 * kMaxBounceSlots * sizeof(uint32_t), st);
   if (e == cudaSuccess) e = timed(Stage::kStart, [&] { return launch_raygen(pb, wt, sms, st); });
+  // a bounce's shadow rays run with the next bounce's queue, or in a launch of their own
+  const bool nee = est == Estimator::kNee, mixed = nee && counters == nullptr;
+  auto shadows = [&](uint32_t b) {
+    return timed(Stage::kTrace, [&] { return launch_trace_shadow(pb, wt, sq, b, sms, st); });
+  };
   for (uint32_t b = 0; b <= max_bounces && e == cudaSuccess; ++b) {
-    if (groups && b >= 1) {
-      e = paths(b);
-      if (b == last) return e;
-    }
-    if (e == cudaSuccess)
-      e = timed(Stage::kTrace, [&] { return launch_trace_wave(pb, wt, single_scene, b, ray_total, sms, st, counters); });
+    const bool to_end = groups && b == last;
+    if (groups) wt.group_limit = to_end ? 0xFFFFFFFFu : kGroupPaths;
+    if (!to_end || mixed)
+      e = timed(Stage::kTrace, [&] {
+        return launch_trace_wave(pb, wt, single_scene, b, mixed ? &sq : nullptr, ray_total, sms, st, counters);
+      });
+    if (e == cudaSuccess && groups && b >= 1) e = paths(b);  // after the shadow rays: it goes on from their sums
+    if (to_end) return e;
     if (e == cudaSuccess)
       e = timed(Stage::kShade, [&] {
         return est == Estimator::kCache ? launch_shade_cache(pb, wt, cw, b, sms, st)
-               : est == Estimator::kNee ? launch_shade_nee(pb, wt, sq, b, sms, st)
+               : nee                    ? launch_shade_nee(pb, wt, sq, b, sms, st)
                                         : launch_shade(pb, wt, b, sms, st);
       });
-    if (e == cudaSuccess && est == Estimator::kNee)
-      e = timed(Stage::kTrace, [&] { return launch_trace_shadow(pb, wt, sq, b, sms, st); });
+    if (e == cudaSuccess && nee && (!mixed || b == max_bounces)) e = shadows(b);
   }
   return e;
 }
