@@ -182,8 +182,10 @@ struct TraceState {
   V3 wo, wd;
   V3 ro, rd, rinv;
   float t_hit;
+  float next_d;                  // have_node: distance of the pending node
   int sp, blas_base;
   uint32_t cur_inst, node, iter, status;
+  uint32_t leaf_mask, leaf_base; // slots of the last node still to test: slot k is record leaf_base + k
   bool in_blas, have_node;
 };
 
@@ -207,6 +209,8 @@ __device__ __forceinline__ void trace_begin(TraceState& t, uint2* stack, const D
   // triangle comparison of the reference fails on NaN; the box test below relies on it)
   const float fin = fabsf(wo.x) + fabsf(wo.y) + fabsf(wo.z) + fabsf(wd.x) + fabsf(wd.y) + fabsf(wd.z);
   t.have_node = s.has_tlas != 0u && fin <= 3.4028235e38f;
+  t.next_d = 0.0f;
+  t.leaf_mask = t.leaf_base = 0;
   t.iter = 0;
 }
 
@@ -303,6 +307,16 @@ struct SharedStack {
   }
 };
 
+// Lane refill: a step goes on to its lanes' further leaf slots only while this many lanes have one.  The
+// others keep theirs for the next step, where they share the pass with the leaves that other lanes
+// reach meanwhile; testing every slot at once, most passes ran with two or three lanes.  1 (all slots) /
+// 3 / 6 / 9 / 12 lanes / one pass per step: scattered any hit on the 1M-triangle soup 4.52 / 4.00 / 3.82
+// / 3.82 / 3.83 / 3.75 ms, closest (1M rays) 1.54 / 1.42 / 1.37 / 1.37 / 1.38 / 1.40, 1920x1080 at
+// 64 spp 105.5 / 101.6 / 101.6 / 101.7 / 101.6 / 103.0, 1013x571 at 3 spp with NEE 3.66 / 3.59 / 3.58 /
+// 3.59 / 3.59 / 3.69.  Whole-warp chunks test all slots: their lanes reach the same leaves together
+// (camera rays on the soup 2.53, with one pass per step 2.97).
+constexpr int kLeafLanes = 6;
+
 // Work counters of the instrumented traversal (kCount instantiations only): what the device
 // layout fetches per ray - 80 bytes of the wide nodes of the TLAS and the BLASes, the triangles of
 // leaf slots (80 bytes for one or two), 64-byte instance records - and the 8-byte stack entries pushed (each later popped);
@@ -319,7 +333,8 @@ __device__ __forceinline__ bool lowest_active(uint32_t mask) {
 }
 
 // Bound by instruction issue and the ALU pipe for camera rays (75% / 75% of peak, 22 of 32 lanes
-// active) and by latency and divergence for secondary rays (66%, 16 of 32).  What it costs per warp
+// active) and by latency and divergence for secondary rays (66%, 16 of 32).  Run twice, the leaf tests
+// add 16% to the 1080p frame (51% to scattered rays in the soup), the sort 4%, the pushes 2%.  What it costs per warp
 // step is its instructions, most of them not in the box tests: a slot's triangles are tested two at a
 // time (triangle_pair_test), the box tests take a child's near and far plane of an axis in one packed
 // FMA, and a hit child's stack entry is one addition (inner children come first in a node, so the slot
@@ -335,32 +350,37 @@ __device__ __forceinline__ bool lowest_active(uint32_t mask) {
 template <bool kAny, bool kCount, class World, class Stack>
 __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, const DevScene& s, TraceCount* cnt,
                                            const World& wr) {
-  if (t.iter > kIterationCap) {
-    t.status |= kStatusIterationCap;
-    return false;
-  }
-  ++t.iter;
   V3 &ro = t.ro, &rd = t.rd, &rinv = t.rinv;
-  float& h_t = t.t_hit;
+  float &h_t = t.t_hit, &next_d = t.next_d;
   int &sp = t.sp, &blas_base = t.blas_base;
   bool &in_blas = t.in_blas, &have_node = t.have_node;
-  uint32_t &cur_inst = t.cur_inst, &node = t.node, &status = t.status;
-  if (!have_node) {
-    bool done = false;
-    for (;;) {
-      if (in_blas && sp == blas_base) {  // BLAS finished: back to the world ray
-        in_blas = false;
-        const V3 wd = wr.d();
-        ro = wr.o(); rd = wd;
-        rinv = wr.inv();
+  uint32_t &cur_inst = t.cur_inst, &node = t.node, &status = t.status, &leaf_mask = t.leaf_mask;
+  if (!Stack::kScattered || leaf_mask == 0u) {  // else the last node's leaf slots come first
+    if (t.iter > kIterationCap) {
+      status |= kStatusIterationCap;
+      return false;
+    }
+    ++t.iter;
+    if (have_node && next_d >= h_t) have_node = false;  // a leaf was closer than the pending node
+    if (!have_node) {
+      // The next entry nearer than the hit.  The loop only finds it; what the entry needs is done once
+      // after the loop by all lanes together, whichever pass they left it in: the world ray is brought
+      // back only for a TLAS node, an instance's ray is made from it directly.
+      bool left = false;  // a BLAS was finished on the way
+      uint2 e = make_uint2(0u, 0u);
+      bool found = false;
+      while (!found) {
+        if (in_blas && sp == blas_base) {
+          in_blas = false;
+          left = true;
+        }
+        if (sp == 0) break;
+        --sp;
+        e = stack.get(sp);
+        found = __uint_as_float(e.y & ~7u) < h_t;  // raytracing_sw.wgsl:197,271
       }
-      if (sp == 0) {
-        done = true;
-        break;
-      }
-      --sp;
-      const uint2 e = stack.get(sp);
-      if (__uint_as_float(e.y & ~7u) >= h_t) continue;  // raytracing_sw.wgsl:197,271
+      if (!found) return false;
+      node = e.x;
       if (!in_blas && (e.x & kInstanceBit)) {
         // enter an instance: transform the world ray (raytracing_sw.wgsl:202-206)
         if (kCount) ++cnt->insts;
@@ -378,150 +398,152 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
         cur_inst = f2u(r3.y);
         in_blas = true;
         blas_base = sp;
-      } else {
-        node = e.x;
+      } else if (left) {  // back to the world ray
+        ro = wr.o();
+        rd = wr.d();
+        rinv = wr.inv();
       }
-      break;
     }
-    if (done) return false;
-  }
-  have_node = false;
+    have_node = false;
 
-  // ---- one 8-wide node: quantised slab tests of all children ----
-  if (kCount) {
-    ++(in_blas ? cnt->blas_nodes : cnt->tlas_nodes);
-    const uint32_t together = __activemask();
-    if (lowest_active(together)) {
-      ++cnt->warp_steps;
-      cnt->lane_steps += (uint32_t)__popc(together);
+    // ---- one 8-wide node: quantised slab tests of all children ----
+    if (kCount) {
+      ++(in_blas ? cnt->blas_nodes : cnt->tlas_nodes);
+      const uint32_t together = __activemask();
+      if (lowest_active(together)) {
+        ++cnt->warp_steps;
+        cnt->lane_steps += (uint32_t)__popc(together);
+      }
     }
-  }
-  const float4* np = (in_blas ? s.blas_wide : s.tlas_wide) + 6 * (size_t)node;
-  const F8 w0 = ld8(np), w1 = ld8(np + 2);
-  const float4 q0 = w0.a, q2 = w1.a, q3 = w1.b, q4 = ld4(np + 4);
-  const uint2 q1 = make_uint2(f2u(w0.b.x), f2u(w0.b.y));
-  const uint32_t eb = f2u(q0.w);
-  const float ax = __uint_as_float((eb & 0xFFu) << 23) * rinv.x;
-  const float ay = __uint_as_float(((eb >> 8) & 0xFFu) << 23) * rinv.y;
-  const float az = __uint_as_float(((eb >> 16) & 0xFFu) << 23) * rinv.z;
-  const float bx = (q0.x - ro.x) * rinv.x, by = (q0.y - ro.y) * rinv.y, bz = (q0.z - ro.z) * rinv.z;
-  // A plane byte q is read as the float F = 2^15 + q (one byte permute: bytes 0, q, 0, 0x47)
-  // and its distance taken as fma(F, a, b - 2^15 a), one rounding more than fma(q, a, b): the
-  // folded constant differs from b - 2^15 a by at most 2^-24 (|b| + 2^15 |a|), so each plane's
-  // distance lies within e = 2^-24 (3 |b| + (2^15 + 510) |a|) of fma(q, a, b).  Near-plane
-  // constants are lowered and far-plane constants raised by d = |a| / 128 + |b| / 2^19 per
-  // axis.  For every plane t = b + q a of the node (|t| <= |b| + 255 |a|) the margin covers
-  // the fold (e <= 1.8e-7 |b| + 0.002 |a|), the approximate reciprocal (<= 2^-22 |t|) and the
-  // rounding of the plane evaluation against the exact reference box (4e-7 |t|): together
-  // at most 8.2e-7 |b| + 0.0022 |a| <= d, so a box never rejects a ray the reference box
-  // accepts.
-  const float dx = fmaf(fabsf(ax), 0.0078125f, fabsf(bx) * 1.9073486328125e-6f);
-  const float dy = fmaf(fabsf(ay), 0.0078125f, fabsf(by) * 1.9073486328125e-6f);
-  const float dz = fmaf(fabsf(az), 0.0078125f, fabsf(bz) * 1.9073486328125e-6f);
-  const float cx = fmaf(-32768.0f, ax, bx), cy = fmaf(-32768.0f, ay, by), cz = fmaf(-32768.0f, az, bz);
-  const float cnx = cx - dx, cfx = cx + dx, cny = cy - dy, cfy = cy + dy, cnz = cz - dz, cfz = cz + dz;
-  const uint32_t child_base = q1.x, prim_base = q1.y;
-  const uint32_t n_inner = eb >> 28;
-  // near/far planes per axis by the sign of the direction: the near plane of a child is its
-  // low plane where rinv >= 0 (t grows with the quantised coordinate), else its high plane
-  const bool pxs = rinv.x >= 0.0f, pys = rinv.y >= 0.0f, pzs = rinv.z >= 0.0f;
-  const uint32_t nx0 = pxs ? f2u(q2.x) : f2u(q3.z), nx1 = pxs ? f2u(q2.y) : f2u(q3.w);
-  const uint32_t fx0 = pxs ? f2u(q3.z) : f2u(q2.x), fx1 = pxs ? f2u(q3.w) : f2u(q2.y);
-  const uint32_t ny0 = pys ? f2u(q2.z) : f2u(q4.x), ny1 = pys ? f2u(q2.w) : f2u(q4.y);
-  const uint32_t fy0 = pys ? f2u(q4.x) : f2u(q2.z), fy1 = pys ? f2u(q4.y) : f2u(q2.w);
-  const uint32_t nz0 = pzs ? f2u(q3.x) : f2u(q4.z), nz1 = pzs ? f2u(q3.y) : f2u(q4.w);
-  const uint32_t fz0 = pzs ? f2u(q4.z) : f2u(q3.x), fz1 = pzs ? f2u(q4.w) : f2u(q3.y);
-  // a child is hit when max(tn, 0) <= min(tf, the largest float below the closest hit)
-  const float t_below = __uint_as_float(f2u(h_t) - 1u);  // h_t > 0
-  // a child's near and far plane of an axis in one packed FMA
-  const F2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
-  const F2 cx2 = pack2(cnx, cfx), cy2 = pack2(cny, cfy), cz2 = pack2(cnz, cfz);
-  uint32_t key[8];
-  uint32_t hits = 0;
+    const float4* np = (in_blas ? s.blas_wide : s.tlas_wide) + 6 * (size_t)node;
+    const F8 w0 = ld8(np), w1 = ld8(np + 2);
+    const float4 q0 = w0.a, q2 = w1.a, q3 = w1.b, q4 = ld4(np + 4);
+    const uint2 q1 = make_uint2(f2u(w0.b.x), f2u(w0.b.y));
+    const uint32_t eb = f2u(q0.w);
+    const float ax = __uint_as_float((eb & 0xFFu) << 23) * rinv.x;
+    const float ay = __uint_as_float(((eb >> 8) & 0xFFu) << 23) * rinv.y;
+    const float az = __uint_as_float(((eb >> 16) & 0xFFu) << 23) * rinv.z;
+    const float bx = (q0.x - ro.x) * rinv.x, by = (q0.y - ro.y) * rinv.y, bz = (q0.z - ro.z) * rinv.z;
+    // A plane byte q is read as the float F = 2^15 + q (one byte permute: bytes 0, q, 0, 0x47)
+    // and its distance taken as fma(F, a, b - 2^15 a), one rounding more than fma(q, a, b): the
+    // folded constant differs from b - 2^15 a by at most 2^-24 (|b| + 2^15 |a|), so each plane's
+    // distance lies within e = 2^-24 (3 |b| + (2^15 + 510) |a|) of fma(q, a, b).  Near-plane
+    // constants are lowered and far-plane constants raised by d = |a| / 128 + |b| / 2^19 per
+    // axis.  For every plane t = b + q a of the node (|t| <= |b| + 255 |a|) the margin covers
+    // the fold (e <= 1.8e-7 |b| + 0.002 |a|), the approximate reciprocal (<= 2^-22 |t|) and the
+    // rounding of the plane evaluation against the exact reference box (4e-7 |t|): together
+    // at most 8.2e-7 |b| + 0.0022 |a| <= d, so a box never rejects a ray the reference box
+    // accepts.
+    const float dx = fmaf(fabsf(ax), 0.0078125f, fabsf(bx) * 1.9073486328125e-6f);
+    const float dy = fmaf(fabsf(ay), 0.0078125f, fabsf(by) * 1.9073486328125e-6f);
+    const float dz = fmaf(fabsf(az), 0.0078125f, fabsf(bz) * 1.9073486328125e-6f);
+    const float cx = fmaf(-32768.0f, ax, bx), cy = fmaf(-32768.0f, ay, by), cz = fmaf(-32768.0f, az, bz);
+    const float cnx = cx - dx, cfx = cx + dx, cny = cy - dy, cfy = cy + dy, cnz = cz - dz, cfz = cz + dz;
+    const uint32_t child_base = q1.x, prim_base = q1.y;
+    const uint32_t n_inner = eb >> 28;
+    // near/far planes per axis by the sign of the direction: the near plane of a child is its
+    // low plane where rinv >= 0 (t grows with the quantised coordinate), else its high plane
+    const bool pxs = rinv.x >= 0.0f, pys = rinv.y >= 0.0f, pzs = rinv.z >= 0.0f;
+    const uint32_t nx0 = pxs ? f2u(q2.x) : f2u(q3.z), nx1 = pxs ? f2u(q2.y) : f2u(q3.w);
+    const uint32_t fx0 = pxs ? f2u(q3.z) : f2u(q2.x), fx1 = pxs ? f2u(q3.w) : f2u(q2.y);
+    const uint32_t ny0 = pys ? f2u(q2.z) : f2u(q4.x), ny1 = pys ? f2u(q2.w) : f2u(q4.y);
+    const uint32_t fy0 = pys ? f2u(q4.x) : f2u(q2.z), fy1 = pys ? f2u(q4.y) : f2u(q2.w);
+    const uint32_t nz0 = pzs ? f2u(q3.x) : f2u(q4.z), nz1 = pzs ? f2u(q3.y) : f2u(q4.w);
+    const uint32_t fz0 = pzs ? f2u(q4.z) : f2u(q3.x), fz1 = pzs ? f2u(q4.w) : f2u(q3.y);
+    // a child is hit when max(tn, 0) <= min(tf, the largest float below the closest hit)
+    const float t_below = __uint_as_float(f2u(h_t) - 1u);  // h_t > 0
+    // a child's near and far plane of an axis in one packed FMA
+    const F2 ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+    const F2 cx2 = pack2(cnx, cfx), cy2 = pack2(cny, cfy), cz2 = pack2(cnz, cfz);
+    uint32_t key[8];
+    uint32_t hits = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    // byte k of the plane words as the float 2^15 + q: bits 0x4700qq00
-    const uint32_t sel = 0x7404u + ((uint32_t)(k & 3) << 4);
-    auto planes = [&](uint32_t n0, uint32_t n1, uint32_t f0, uint32_t f1) {
-      return pack2(__byte_perm(k < 4 ? n0 : n1, 0x47000000u, sel), __byte_perm(k < 4 ? f0 : f1, 0x47000000u, sel));
-    };
-    const float2 tx = unpack2(fma2(planes(nx0, nx1, fx0, fx1), ax2, cx2));
-    const float2 ty = unpack2(fma2(planes(ny0, ny1, fy0, fy1), ay2, cy2));
-    const float2 tz = unpack2(fma2(planes(nz0, nz1, fz0, fz1), az2, cz2));
-    const float lo = fmaxf(fmaxf(fmaxf(tx.x, ty.x), tz.x), 0.0f);
-    const float hi = fminf(fminf(fminf(tx.y, ty.y), tz.y), t_below);
-    if (lo <= hi) hits |= 1u << k;
-    key[k] = (f2u(lo) & ~7u) | (uint32_t)k;
-  }
-  hits &= (1u << ((eb >> 24) & 15u)) - 1u;
-  const uint32_t inner = in_blas ? (1u << n_inner) - 1u : 0xFFu;  // children that are visited, not tested
-  uint32_t leaf_mask = hits & ~inner;
-  const uint32_t push_mask = hits & inner;
-  const int n_push = __popc(push_mask);
+    for (int k = 0; k < 8; ++k) {
+      // byte k of the plane words as the float 2^15 + q: bits 0x4700qq00
+      const uint32_t sel = 0x7404u + ((uint32_t)(k & 3) << 4);
+      auto planes = [&](uint32_t n0, uint32_t n1, uint32_t f0, uint32_t f1) {
+        return pack2(__byte_perm(k < 4 ? n0 : n1, 0x47000000u, sel), __byte_perm(k < 4 ? f0 : f1, 0x47000000u, sel));
+      };
+      const float2 tx = unpack2(fma2(planes(nx0, nx1, fx0, fx1), ax2, cx2));
+      const float2 ty = unpack2(fma2(planes(ny0, ny1, fy0, fy1), ay2, cy2));
+      const float2 tz = unpack2(fma2(planes(nz0, nz1, fz0, fz1), az2, cz2));
+      const float lo = fmaxf(fmaxf(fmaxf(tx.x, ty.x), tz.x), 0.0f);
+      const float hi = fminf(fminf(fminf(tx.y, ty.y), tz.y), t_below);
+      if (lo <= hi) hits |= 1u << k;
+      key[k] = (f2u(lo) & ~7u) | (uint32_t)k;
+    }
+    hits &= (1u << ((eb >> 24) & 15u)) - 1u;
+    const uint32_t inner = in_blas ? (1u << n_inner) - 1u : 0xFFu;  // children that are visited, not tested
+    leaf_mask = hits & ~inner;
+    t.leaf_base = prim_base - n_inner;
+    const uint32_t push_mask = hits & inner;
+    const int n_push = __popc(push_mask);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) key[k] = (push_mask & (1u << k)) ? key[k] : 0xFFFFFFFFu;
+    for (int k = 0; k < 8; ++k) key[k] = (push_mask & (1u << k)) ? key[k] : 0xFFFFFFFFu;
 
-  // The hit children are ordered and pushed before the node's leaf triangles are tested:
-  // the keys' registers are free again during the triangle loads (measured 1.6% faster than
-  // testing leaves first).  A leaf hit closer than the child visited next drops that child.
-  float next_d = 0.0f;
-  // ---- order hit children near to far (19-comparator network) ----
+    // The hit children are ordered and pushed before the node's leaf triangles are tested:
+    // the keys' registers are free again during the triangle loads (measured 1.6% faster than
+    // testing leaves first).  A leaf hit closer than the child visited next drops that child.
+    // ---- order hit children near to far (19-comparator network) ----
 #define NB_CX(i, j)                                  \
 {                                                  \
-  const uint32_t lo_ = min(key[i], key[j]);        \
-  key[j] = max(key[i], key[j]);                    \
-  key[i] = lo_;                                    \
-}
-  if (n_push > 0) {
-    if (!Stack::kScattered && n_push == 1) {  // the single hit child: no sort
+    const uint32_t lo_ = min(key[i], key[j]);        \
+    key[j] = max(key[i], key[j]);                    \
+    key[i] = lo_;                                    \
+  }
+    if (n_push > 0) {
+      if (!Stack::kScattered && n_push == 1) {  // the single hit child: no sort
 #pragma unroll
-      for (int k = 1; k < 8; ++k) key[0] = min(key[0], key[k]);
-    } else {
-      NB_CX(0, 2) NB_CX(1, 3) NB_CX(4, 6) NB_CX(5, 7)
-      NB_CX(0, 4) NB_CX(1, 5) NB_CX(2, 6) NB_CX(3, 7)
-      NB_CX(0, 1) NB_CX(2, 3) NB_CX(4, 5) NB_CX(6, 7)
-      NB_CX(2, 4) NB_CX(3, 5)
-      NB_CX(1, 4) NB_CX(3, 6)
-      NB_CX(1, 2) NB_CX(3, 4) NB_CX(5, 6)
-    }
-    // a child's stack entry: node or instance index and its key (its slot in the low 3 bits)
-    const uint32_t inst_base = kInstanceBit + prim_base - n_inner;
-    auto entry = [&](uint32_t kk) {
-      const uint32_t slot = kk & 7u;
-      return make_uint2((slot < n_inner ? child_base : inst_base) + slot, kk);
-    };
-    // far to near, the nearest at top; the nearest inner child is visited next without a push
-    const int top = sp + n_push - 1;
-    const uint2 first = entry(key[0]);
-    have_node = !(first.x & kInstanceBit);
-    if (top < Stack::kFast) {
-      uint2* at = stack.fast(top);
+        for (int k = 1; k < 8; ++k) key[0] = min(key[0], key[k]);
+      } else {
+        NB_CX(0, 2) NB_CX(1, 3) NB_CX(4, 6) NB_CX(5, 7)
+        NB_CX(0, 4) NB_CX(1, 5) NB_CX(2, 6) NB_CX(3, 7)
+        NB_CX(0, 1) NB_CX(2, 3) NB_CX(4, 5) NB_CX(6, 7)
+        NB_CX(2, 4) NB_CX(3, 5)
+        NB_CX(1, 4) NB_CX(3, 6)
+        NB_CX(1, 2) NB_CX(3, 4) NB_CX(5, 6)
+      }
+      // a child's stack entry: node or instance index and its key (its slot in the low 3 bits)
+      const uint32_t inst_base = kInstanceBit + prim_base - n_inner;
+      auto entry = [&](uint32_t kk) {
+        const uint32_t slot = kk & 7u;
+        return make_uint2((slot < n_inner ? child_base : inst_base) + slot, kk);
+      };
+      // far to near, the nearest at top; the nearest inner child is visited next without a push
+      const int top = sp + n_push - 1;
+      const uint2 first = entry(key[0]);
+      have_node = !(first.x & kInstanceBit);
+      if (top < Stack::kFast) {
+        uint2* at = stack.fast(top);
 #pragma unroll
-      for (int k = 1; k < 8; ++k)
-        if (k < n_push) at[-k * Stack::kStride] = entry(key[k]);
-      if (!have_node) at[0] = first;
-      sp = have_node ? top : top + 1;
-    } else {
-      // one by one, the last ones only as far as they fit
+        for (int k = 1; k < 8; ++k)
+          if (k < n_push) at[-k * Stack::kStride] = entry(key[k]);
+        if (!have_node) at[0] = first;
+        sp = have_node ? top : top + 1;
+      } else {
+        // one by one, the last ones only as far as they fit
 #pragma unroll
-      for (int k = 7; k >= 0; --k) {
-        if (k >= n_push || (k == 0 && have_node)) continue;
-        if (sp < kStackSize) stack.put(sp++, entry(key[k]));
-        else status |= kStatusStackOverflow;
+        for (int k = 7; k >= 0; --k) {
+          if (k >= n_push || (k == 0 && have_node)) continue;
+          if (sp < kStackSize) stack.put(sp++, entry(key[k]));
+          else status |= kStatusStackOverflow;
+        }
+      }
+      if (kCount) cnt->pushes += (uint32_t)(n_push - (have_node ? 1 : 0));
+      if (have_node) {
+        node = first.x;
+        next_d = __uint_as_float(first.y & ~7u);
       }
     }
-    if (kCount) cnt->pushes += (uint32_t)(n_push - (have_node ? 1 : 0));
-    if (have_node) {
-      node = first.x;
-      next_d = __uint_as_float(first.y & ~7u);
-    }
-  }
 #undef NB_CX
+  }
   if (kCount) {
     const uint32_t together = __activemask();
     uint32_t n_tris = 0;
-    for (uint32_t lm = leaf_mask; lm; lm &= lm - 1)
-      n_tris += f2u(ld4(s.tris + 6 * (size_t)(prim_base + (uint32_t)(__ffs(lm) - 1) - n_inner) + 4).w) == 0xFFFFFFFFu ? 1u : 2u;
+    if (leaf_mask) {
+      const uint32_t k = (uint32_t)(__ffs(leaf_mask) - 1);
+      n_tris = f2u(ld4(s.tris + 6 * (size_t)(t.leaf_base + k) + 4).w) == 0xFFFFFFFFu ? 1u : 2u;
+    }
     cnt->tris += n_tris;
     const uint32_t with_leaves = __ballot_sync(together, leaf_mask != 0u);
     const uint32_t most = __reduce_max_sync(together, n_tris);
@@ -531,12 +553,13 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
       cnt->leaf_trips += most;
     }
   }
-  // ---- BLAS leaves: Moller-Trumbore (raytracing_sw.wgsl:51-78, 274-286) ----
+  // ---- BLAS leaf slots: Moller-Trumbore (raytracing_sw.wgsl:51-78, 274-286), all of the node's or as
+  // many as enough lanes have (kLeafLanes) ----
   while (leaf_mask) {
     const uint32_t k = (uint32_t)(__ffs(leaf_mask) - 1);
     leaf_mask &= leaf_mask - 1;
     bool found = false;
-    triangle_pair_test(ro, rd, s.tris + 6 * (size_t)(prim_base + k - n_inner), h_t,
+    triangle_pair_test(ro, rd, s.tris + 6 * (size_t)(t.leaf_base + k), h_t,
                        [&](float t, float u, float v, uint32_t tri) {
                          if (kAny && found) return;  // any hit: the first
                          h_t = t;
@@ -545,9 +568,8 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
                          found = true;
                        });
     if (kAny && found) return false;
+    if (Stack::kScattered && __popc(__ballot_sync(__activemask(), leaf_mask != 0u)) < kLeafLanes) break;
   }
-
-  if (have_node && next_d >= h_t) have_node = false;  // a leaf above is closer than the next node
   return true;
 }
 
