@@ -131,7 +131,7 @@ struct GroupTrace {
       __syncwarp();  // the entries are read before the pushes below
     }
 
-    // ---- this lane's child: the slab test of trace_step ----
+    // ---- this lane's child: the slab test of trace_step, with any-hit queries' offset ----
     // plane bytes (WideNode): lo x, y, z at 32, 40, 48 and hi x, y, z at 56, 64, 72, one per child;
     // the near plane is the low one where the direction is positive
     float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
