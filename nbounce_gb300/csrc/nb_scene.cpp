@@ -702,7 +702,14 @@ struct Collapser {
         if (ok) break;
       }
       w->p[k] = p;
-      w->e[k] = (uint8_t)(e + 127);
+      const float step = (float)std::ldexp(1.0, e);
+      if (k < 2) {
+        w->step[k] = step;
+      } else {
+        uint32_t u;
+        std::memcpy(&u, &step, sizeof(u));
+        w->bits |= u;
+      }
     }
   }
 
@@ -799,7 +806,7 @@ struct Collapser {
       WideNode w{};
       std::vector<Item> slots;
       w.child_base = (uint32_t)out->size();
-      w.prim_base = (uint32_t)(prim_order->size() / max_leaf);
+      const uint32_t first_leaf = (uint32_t)(prim_order->size() / max_leaf);
       uint32_t n_inner = 0;
       for (const int32_t x : items) {
         const Item& it = dp[x].it;
@@ -812,7 +819,8 @@ struct Collapser {
         }
         slots.push_back(it);
       }
-      w.counts = (uint8_t)(slots.size() | n_inner << 4);
+      w.leaf_base = first_leaf - n_inner;
+      w.set_children((uint32_t)slots.size(), n_inner);
       quantise(&w, slots);
       (*out)[self] = w;
     }
@@ -958,7 +966,7 @@ void entry_boxes(const HostScene& s, const std::vector<uint32_t>& tri_order, con
           st.push_back(w.child_base + c);
           continue;
         }
-        const size_t pair = w.prim_base + c - w.n_inner();
+        const size_t pair = w.leaf_base + c;
         for (int j = 0; j < 2; ++j) {
           const uint32_t t = tri_order[2 * pair + j];
           if (t == kNoPrim) continue;
@@ -1077,7 +1085,7 @@ int to_device_layout(HostScene* s) {
     s->wblas_root.push_back(node_off);
     for (WideNode w : wide[k]) {
       w.child_base += node_off;
-      w.prim_base += prim_off;
+      w.leaf_base += prim_off;
       s->wblas.push_back(w);
     }
     tri_order.insert(tri_order.end(), order[k].begin(), order[k].end());
