@@ -555,9 +555,16 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
       have_node = !(first.x & kInstanceBit);
       if (top < Stack::kFast) {
         uint2* at = stack.fast(top);
+        // (the branch over the last four: 1920x1080 at 64 spp 92.6 -> 91.0 ms, camera rays 2.29 -> 2.26;
+        // over the last five and three 91.0 and 91.2, 2.23 and 2.25, scattered any hit 3.62, 3.58 against 3.59)
 #pragma unroll
-        for (int k = 1; k < 8; ++k)
+        for (int k = 1; k < 4; ++k)
           if (k < n_push) at[-k * Stack::kStride] = entry(key[k]);
+        if (n_push > 4) {
+#pragma unroll
+          for (int k = 4; k < 8; ++k)
+            if (k < n_push) at[-k * Stack::kStride] = entry(key[k]);
+        }
         if (!have_node) at[0] = first;
         sp = have_node ? top : top + 1;
       } else {
