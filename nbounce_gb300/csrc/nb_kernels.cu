@@ -277,11 +277,12 @@ __device__ __forceinline__ void trace_begin(TraceState& t, uint2* stack, const D
 constexpr int kWorldFloats = 9 * 32;
 constexpr int kTraceWarps = 4;  // every traversal kernel runs blocks of 128 threads
 constexpr int kTraceThreads = 32 * kTraceWarps;
-// Blocks per SM of the traversal kernels: with lane refill 7 (72 registers), whole-warp chunks 6 (80).
-// The packed test of a slot's two triangles needs the registers; with one block more the kernels spill
-// 40-140 bytes.  1920x1080 at 64 spp (1.2M triangles) / scattered any hit and camera rays on the
-// 1M-triangle soup, refill and chunk blocks 9+7: 118.0 / 6.06 / 2.54 ms, 8+7: 115.7 / 5.67 / 2.54,
-// 7+6: 110.4 / 5.02 / 2.53, 6+5: 114.4 / 5.05 / 2.66.
+// Blocks per SM of the traversal kernels: with lane refill 7 (72 registers), whole-warp chunks 6 (80), of
+// closest-hit queries 7.  Camera grids of 2048x2048 with 6 / 7: closest hits on soups of 1M, 200K and 20K
+// triangles 2.28 / 2.23, 2.07 / 2.03 and 0.72 / 0.71 ms, on the instanced scene 1.35 / 1.32; any hits
+// 2.02 / 2.03, 2.04 / 2.06, 0.74 / 0.75 and 1.11 / 1.14, and a render's camera rays with 7 no faster than with
+// 6.  1920x1080 at 64 spp and scattered any hit, refill and chunk blocks 8+7: 103.5 and 4.79 ms, 7+6: 90.9
+// and 3.59, 6+5: 94.4 and 3.77.
 constexpr int kRefillBlocks = 7, kChunkBlocks = 6;
 struct WorldRegs {
   const TraceState& t;
@@ -706,7 +707,7 @@ namespace nbd {
 // kRefill: lanes refill as they finish (trace_refill), for rays whose neighbours in the array
 // are unrelated; else each warp traces 32 consecutive rays to the end.
 template <bool kAny, bool kRefill>
-__global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kChunkBlocks)
+__global__ void __launch_bounds__(kTraceThreads, kRefill || !kAny ? kRefillBlocks : kChunkBlocks)
     k_trace_rays(DevScene s, const float4* __restrict__ rays, uint32_t n, float4* __restrict__ hits,
                  uint32_t* __restrict__ inst, uint32_t* __restrict__ fetch, uint32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
