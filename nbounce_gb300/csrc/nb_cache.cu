@@ -10,8 +10,8 @@
 // Kernels (mma.sync m16n8k16, BF16 operands, FP32 accumulation; weights resident in shared
 // memory as 336 rows x 64 inputs, rows padded to 72 elements so that ldmatrix is
 // conflict-free):
-//   k_cache_infer_tc tcgen05.mma (5th-generation tensor cores): operands in shared memory,
-//                    FP32 accumulators in tensor memory, 4 groups of 128 rows per CTA
+//   k_cache_infer_tc tcgen05.mma (5th-generation tensor cores): weights in shared memory,
+//                    activations and FP32 accumulators in tensor memory, 8 groups of 128 rows per CTA
 //   k_cache_infer_*  mma.sync: one warp evaluates 32 rows, the activations never leave
 //                    registers (the C fragment of layer l, ReLU'd and packed to BF16, is the A
 //                    fragment of layer l + 1)

@@ -382,8 +382,9 @@ __device__ __forceinline__ bool lowest_active(uint32_t mask) {
   return (threadIdx.x & 31u) == (uint32_t)(__ffs(mask) - 1);
 }
 
-// Bound by instruction issue and the ALU pipe for camera rays (75% / 75% of peak, 22 of 32 lanes
-// active) and by latency and divergence for secondary rays (66%, 16 of 32).  Run twice, the leaf tests
+// Bound by instruction issue, latency and divergence: the schedulers issue in 72% of cycles for camera rays
+// (ALU pipe 60% of its peak, 20 of 32 lanes active) and 73% for secondary rays (56%, 16 of 32; the
+// benchmark scene at 480x270, 64 spp).  Run twice, the leaf tests
 // add 16% to the 1080p frame (51% to scattered rays in the soup), the sort 4%, the pushes 2%.  What it costs per warp
 // step is its instructions, most of them not in the box tests: a slot's triangles are tested two at a
 // time (triangle_pair_test), the box tests take a child's near and far plane of an axis in one packed
