@@ -916,7 +916,7 @@ int nb_trace_rays(const nb_scene* scene, const float* rays, size_t n, uint32_t f
   return NB_OK;
 }
 
-// nb_trace_rays_host through the scene's page-locked buffer (1 <= n <= kGroupPaths)
+// nb_trace_rays_host through the scene's page-locked buffer (1 <= n <= kPinnedRays)
 static int trace_rays_pinned(const nb_scene* scene, const float* rays, size_t n, uint32_t flags, float* hits,
                              uint32_t* instances, cudaStream_t st) {
   HostQuery& q = scene->host_query;
@@ -960,7 +960,7 @@ int nb_trace_rays_host(const nb_scene* scene, const float* rays, size_t n, uint3
   cudaStream_t st = (cudaStream_t)stream;
   if (flags & ~(uint32_t)(NB_TRACE_ANY | NB_TRACE_INCOHERENT))
     return fail(NB_ERR_INVALID_ARG, "unknown trace flags 0x%x", flags);
-  if (n >= 1 && n <= kGroupPaths) return trace_rays_pinned(scene, rays, n, flags, hits, instances, st);
+  if (n >= 1 && n <= kPinnedRays) return trace_rays_pinned(scene, rays, n, flags, hits, instances, st);
   DeviceArena tmp;
   void *dr = nullptr, *dh = nullptr, *di = nullptr;
   int rc;

@@ -2139,7 +2139,7 @@ cudaError_t launch_trace_rays(const nbd::DevScene& s, const float* rays, uint32_
                               float* hits, uint32_t* inst, uint32_t* fetch, uint32_t* status, int sms,
                               cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  if (n <= kGroupPaths) {
+  if (n <= (refill ? kGroupScattered : kGroupRays)) {
     const void* kernel = any ? (const void*)nbd::k_trace_rays_group<true> : (const void*)nbd::k_trace_rays_group<false>;
     static const int full[2] = {blocks_for((const void*)nbd::k_trace_rays_group<false>, nbd::kGroupThreads, sms),
                                 blocks_for((const void*)nbd::k_trace_rays_group<true>, nbd::kGroupThreads, sms)};

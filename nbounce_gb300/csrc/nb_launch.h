@@ -122,14 +122,17 @@ enum class Estimator { kPlain, kNee, kCache };
 cudaError_t launch_trace_paths(const PathBatch& pb, const WaveTables& wt, Estimator est, const CacheWave& cw,
                                uint32_t bounce, unsigned long long* ray_total, int sms, cudaStream_t st);
 
-// Queues and waves up to this many paths, and nb_trace_rays calls up to this many rays, are traced by
-// 8 lanes per ray.  Such a ray costs ~2.5 times the instructions of a ray per lane, but a node step
-// takes 0.8 us instead of ~2, and a launch is as long as its longest ray until the GPU is full:
-// scattered rays through a 300K-triangle scene take 42 against 95 us (152 rays), 81 / 161 (9,728),
-// 165 / 193 (65,536), 286 / 238 (131,072).  With the paths run to their ends (k_trace_paths), limits
-// of 16K / 32K / 64K / 128K paths: 576x320 at 1 spp 856 / 803 / 772 / 853 us (1573 with per-bounce
-// launches alone), 256x256 at 16 spp 608 / 580 / 570 / 600 us (720), 64x48 at 1 spp 69 us (339).
-constexpr uint32_t kGroupPaths = 1u << 16;
+// Queues and waves up to kGroupPaths paths, and nb_trace_rays calls up to kGroupRays rays
+// (kGroupScattered with NB_TRACE_INCOHERENT), are traced by 8 lanes per ray.  Such a ray costs ~2.5 times the instructions of a ray per lane, but a node step
+// takes 0.8 us instead of ~2, and a launch is as long as its longest ray until the GPU is full.
+// Paths (run to their ends by k_trace_paths), limits of 16K / 24K / 32K / 64K: 160x120 at 1 spp on the
+// instanced scene 320 / 260 / 262 / 260 us, 256x256 514 / 516 / 517 / 642, with NEE 1000 / 1000 / 1194 /
+// 1544, 400x300 626 / 631 / 594 / 679, 576x320 669 / 657 / 653 / 642, 1013x571 at 3 spp with NEE 3025 / 3090 /
+// 3080 / 3348.  Rays, 8 lanes against one, closest hits: camera grids of 16,384 rays on soups of 2K, 20K and
+// 1M triangles 24 / 24, 50 / 58 and 108 / 145 us, of 32,761 rays 33 / 23, 63 / 59 and 156 / 178; 24,025
+// scattered rays 37 / 38, 76 / 92 and 190 / 250, 32,761 44 / 40, 91 / 94 and 218 / 256.
+constexpr uint32_t kGroupPaths = 1u << 15;
+constexpr uint32_t kGroupRays = 1u << 14, kGroupScattered = 3u << 13;
 
 // The launch kinds of a wave (nb_kernel_times)
 enum class Stage { kStart, kTrace, kShade };

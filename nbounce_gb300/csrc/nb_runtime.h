@@ -83,7 +83,8 @@ int parse_dds_cube(const uint8_t* bytes, size_t n, DdsCube* out);
 
 // Page-locked buffer of nb_trace_rays_host: short queries read their rays from it and write their hits
 // into it, so that a call needs no device allocations and no copy commands.  Kept with the scene, at
-// most kGroupPaths rays' worth (3.4 MB); calls on the same scene take turns.
+// most kPinnedRays rays' worth (3.4 MB); calls on the same scene take turns.
+constexpr size_t kPinnedRays = 1u << 16;
 struct HostQuery {
   std::mutex mu;
   char* mem = nullptr;

@@ -9,7 +9,7 @@ from nbounce_gb300 import scenes
 
 pytestmark = pytest.mark.gpu
 
-LIMIT = 65536  # rays up to which a call is traced in groups
+LIMIT = 65536  # above it no call is traced in groups (below 16,384 all are)
 
 
 def _edge_rays(desc, scale, seed):

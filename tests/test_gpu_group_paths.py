@@ -1,7 +1,7 @@
 """Queries and waves that the library traces with 8 lanes per ray against the same ones traced with a
 ray per lane: the hits, images, ray counts and cache weights are the same bits.
 
-A ray per lane is had from a call with more than 65,536 rays, and for renders from the instrumented
+A ray per lane is had from a call with more rays than the limits, and for renders from the instrumented
 traversal (enable_trace_counters), which traces a ray per lane whatever the size."""
 import numpy as np
 import pytest
@@ -11,7 +11,8 @@ from nbounce_gb300 import scenes
 
 pytestmark = pytest.mark.gpu
 
-LIMIT = 65536  # rays and paths up to which a call or a wave is traced in groups
+LIMIT = 65536  # above it no call or wave is traced in groups: 32,768 paths, 16,384 rays, 24,576 scattered ones
+EDGES = (16384, 16385, 24576, 24577, 32768)
 
 
 @pytest.fixture(scope="module")
@@ -42,7 +43,7 @@ def test_few_rays_equal_many(world, kind, any_hit):
     scene = world[kind][0]
     hits, inst = scene.trace_host(rays, any_hit=any_hit, incoherent=True)  # a ray per lane
     assert (hits[:, 0] < 3e38).mean() > 0.05
-    for m in (1, 3, 4, 5, 31, 33, 2431, LIMIT - 1, LIMIT):
+    for m in (1, 3, 4, 5, 31, 33, 2431, *EDGES, LIMIT - 1, LIMIT):
         for incoherent in (False, True):
             h, i = scene.trace_host(rays[:m], any_hit=any_hit, incoherent=incoherent)
             assert np.array_equal(h.view(np.uint32), hits[:m].view(np.uint32)) and np.array_equal(i, inst[:m]), m
@@ -59,14 +60,15 @@ def _render(scene, env, kind, w, h, spp, bounces, nee, rr, per_lane, batch=0):
     return pt.download(), pt.last_stats()
 
 
-# waves around the limits: all bounces in one launch (up to 65,536 paths), from bounce 1 on (twice
+# waves around the limits: all bounces in one launch (up to 32,768 paths), from bounce 1 on (twice
 # that), from later bounces on, and short queues within a larger wave
 @pytest.mark.parametrize("kind,w,h,spp,bounces,nee,rr", [
     ("spheres", 1, 1, 1, 8, False, 0), ("spheres", 3, 5, 1, 0, False, 0), ("instanced", 33, 27, 2, 8, True, 0),
     ("instanced", 255, 257, 1, 8, False, 0), ("instanced", 256, 256, 1, 3, True, 3), ("room", 256, 257, 1, 8, False, 0),
     ("instanced", 257, 256, 1, 8, True, 0), ("spheres", 300, 437, 1, 6, False, 0), ("room", 363, 361, 1, 12, False, 0),
     ("instanced", 511, 513, 1, 8, False, 3), ("spheres", 640, 480, 2, 6, True, 0), ("instanced", 801, 603, 3, 8, True, 0),
-    ("instanced", 801, 603, 3, 8, False, 0)])
+    ("instanced", 801, 603, 3, 8, False, 0), ("instanced", 181, 181, 1, 8, False, 0), ("spheres", 128, 256, 1, 8, True, 0),
+    ("instanced", 127, 259, 1, 8, True, 0), ("room", 129, 255, 1, 8, False, 3)])
 def test_render_equals_ray_per_lane(world, kind, w, h, spp, bounces, nee, rr):
     scene, env = world[kind]
     a, sa = _render(scene, env, kind, w, h, spp, bounces, nee, rr, False)
