@@ -132,7 +132,6 @@ static int upload_scene(nb_scene* s) {
   NB_CUDA(cudaMemset(p, 0, 2 * sizeof(uint32_t)), "cudaMemset");
   // drop device-layout host copies; keep the reference-layout buffers for nb_scene_export
   h.wblas_nodes = h.wblas.size();
-  h.wtlas_nodes = h.wtlas.size();
   std::vector<WideNode>().swap(h.wblas);
   std::vector<WideNode>().swap(h.wtlas);
   std::vector<GpuTriPair>().swap(h.tris);
@@ -275,7 +274,7 @@ int nb_scene_get_info(const nb_scene* s, nb_scene_info* info) {
   info->n_blas_nodes_ref = h.blas.size();
   info->n_tlas_nodes_ref = h.tlas.size();
   info->n_blas_nodes_gpu = s->uploaded ? h.wblas_nodes : h.wblas.size();
-  info->n_tlas_nodes_gpu = s->uploaded ? h.wtlas_nodes : h.wtlas.size();
+  info->n_tlas_nodes_gpu = h.wtlas_nodes;
   info->n_tlas_entries = h.tlas_entries;
   info->device_bytes = s->arena.bytes;
   info->build_ms = h.build_ms;

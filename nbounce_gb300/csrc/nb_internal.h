@@ -54,25 +54,23 @@ struct alignas(16) GpuVAttr {
 };
 // 8-wide node collapsed from the reference's binary tree (96 B).  Child boxes are
 // quantised to 8 bits per plane on a per-axis power-of-two grid anchored at p; the quantised
-// boxes contain the exact ones.  The inner children come first: slot k is the inner child at
-// child_base + k for k < n_inner, and up to n_children the leaf slot at leaf_base + k, modulo 2^32 (a
-// GpuTriPair in a BLAS, a GpuInstTrace in the TLAS).  The masks and the grid steps lie ready for use, in
-// words that the loads bring anyway, because the ALU pipe bounds the traversal: as counts and exponents to
-// shift and mask, 1920x1080 at 64 spp took 94.0 instead of 92.6 ms, camera rays on the 1M-triangle soup
-// 2.33 instead of 2.29.
+// boxes contain the exact ones.  Slot k is the inner child child_base + k or the leaf slot leaf_base + k
+// (a GpuTriPair in a BLAS, a GpuInstTrace in the TLAS), by the mask of inner children and modulo 2^32;
+// which order the slots have, and why: Collapser (nb_scene.cpp).  The masks and the grid steps lie ready
+// for use, in words that the loads bring anyway, because the ALU pipe bounds the traversal: as counts and
+// exponents to shift and mask, 1920x1080 at 64 spp took 94.0 instead of 92.6 ms, camera rays on the
+// 1M-triangle soup 2.33 instead of 2.29.
 struct alignas(32) WideNode {
   float p[3];
-  uint32_t bits;       // children mask | inner children mask << 8 | n_inner << 16 | grid step of z (float bits)
+  uint32_t bits;       // children mask | inner children mask << 8 | grid step of z (float bits)
   uint32_t child_base;
   uint32_t leaf_base;
   float step[2];       // grid steps of x and y, powers of two
   uint8_t qlo_x[8], qlo_y[8], qlo_z[8], qhi_x[8], qhi_y[8], qhi_z[8];
   uint32_t pad[4];
   uint32_t n_children() const { return (uint32_t)__builtin_popcount(bits & 0xFFu); }
-  uint32_t n_inner() const { return bits >> 16 & 15u; }
-  void set_children(uint32_t n, uint32_t n_inner) {
-    bits |= ((1u << n) - 1u) | ((1u << n_inner) - 1u) << 8 | n_inner << 16;
-  }
+  uint32_t inner() const { return bits >> 8 & 0xFFu; }
+  void set_children(uint32_t n, uint32_t inner) { bits |= ((1u << n) - 1u) | inner << 8; }
 };
 static_assert(sizeof(WideNode) == 96, "WideNode");
 constexpr uint32_t kInstanceBit = 0x80000000u;  // TLAS stack entry that names an instance
@@ -92,8 +90,9 @@ struct HostScene {
 
   std::vector<WideNode> wblas, wtlas;  // 8-wide trees; the TLAS root is wtlas[0]
   std::vector<uint32_t> wblas_root;    // per distinct BLAS root: index of its root in wblas
-  size_t wblas_nodes = 0, wtlas_nodes = 0;  // sizes kept after the host copies are dropped
-  size_t tlas_entries = 0;                  // device TLAS leaves (itrace records)
+  size_t wblas_nodes = 0;  // size kept after the host copy is dropped
+  size_t wtlas_nodes = 0;  // TLAS nodes without the gaps between them
+  size_t tlas_entries = 0;                  // device TLAS leaves (itrace records without the gaps)
   bool has_tlas = false;
   std::vector<GpuInstTrace> itrace;
   std::vector<GpuInstShade> ishade;

@@ -71,7 +71,6 @@ struct NodeHead {
   uint32_t bits, child_base, leaf_base;
   float step_x, step_y;
   __device__ __forceinline__ float step_z() const { return __uint_as_float(bits & 0x7F800000u); }
-  __device__ __forceinline__ uint32_t n_inner() const { return bits >> 16 & 15u; }
 };
 __device__ __forceinline__ NodeHead load_head(const float4* node) {
   NodeHead h;
@@ -388,8 +387,8 @@ __device__ __forceinline__ bool lowest_active(uint32_t mask) {
 // add 16% to the 1080p frame (51% to scattered rays in the soup), the sort 4%, the pushes 2%.  What it costs per warp
 // step is its instructions, most of them not in the box tests: a slot's triangles are tested two at a
 // time (triangle_pair_test), the box tests take a child's near and far plane of an axis in one packed
-// FMA, and a hit child's stack entry is one addition (inner children come first in a node, so the slot
-// is the offset) stored at a fixed place below the batch's top.  Against one triangle at a time,
+// FMA, and a hit child's stack entry is one addition (the slot is the offset) stored at a fixed place below
+// the batch's top.  Against one triangle at a time,
 // slot metadata and a branch per pushed child, at the same sizes as above: 1920x1080 at 64 spp 116.6 ->
 // 110.4 ms, camera rays on the soup 2.67 -> 2.53, scattered any hit 5.42 -> 5.02, closest (1M rays)
 // 1.94 -> 1.71 ms.
@@ -545,11 +544,14 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
         NB_CX(1, 4) NB_CX(3, 6)
         NB_CX(1, 2) NB_CX(3, 4) NB_CX(5, 6)
       }
-      // a child's stack entry: node or instance index and its key (its slot in the low 3 bits)
-      const uint32_t n_inner = nh.n_inner(), inst_base = kInstanceBit + nh.leaf_base;
+      // a child's stack entry: node or instance index and its key (its slot in the low 3 bits).  (Which of the
+      // two by the mask, since a TLAS node's slots mix them: 1920x1080 at 64 spp 88.2 ms, camera rays on the
+      // soup 2.25, scattered any hit 3.57.  With the inner children first and a comparison 87.8, 2.23 and 3.57, but
+      // then an inner child came before an instance at the same distance, whatever their places in the tree.)
+      const uint32_t inst_base = kInstanceBit + nh.leaf_base;
       auto entry = [&](uint32_t kk) {
         const uint32_t slot = kk & 7u;
-        return make_uint2((slot < n_inner ? nh.child_base : inst_base) + slot, kk);
+        return make_uint2(((nh.bits & (0x100u << slot)) ? nh.child_base : inst_base) + slot, kk);
       };
       // far to near, the nearest at top; the nearest inner child is visited next without a push
       const int top = sp + n_push - 1;

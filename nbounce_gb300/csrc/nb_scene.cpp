@@ -576,11 +576,16 @@ namespace {
 // Measured on the benchmark frame against the greedy collapse that opens the largest-area item
 // first: 35% fewer BLAS nodes and 3% more rays/s; letting the programme also choose leaf sizes
 // (1 to 3 triangles, with a triangle-test weight) was 0.3-1.5% slower than fixed 2-triangle
-// leaves.  Nodes are emitted breadth-first so the inner children of a node are contiguous,
-// and the primitives of a node's leaf slots are written contiguously, in slot order, into a
-// new primitive order.  Traversal finds the same closest hit: the wide BLAS trees cover the
+// leaves.  Nodes are emitted breadth-first: the child in slot k is node child_base + k if it is an
+// inner one, and leaf slot leaf_base + k of a new primitive order if it is a leaf.  A slot's place
+// decides between children at the same distance (the traversal's sort keys end in it), so the slots
+// keep the order in which the cover lists them.  A BLAS may put a node's inner children first without
+// touching that, because its leaf slots are never pushed: only inner children compete, and both arrays
+// stay dense.  TLAS leaves are pushed among the inner children, so there the slots stay as listed and
+// the arrays have gaps: a node's inner children span the slots from its first to its last one, and so
+// do its leaves.  Traversal finds the same closest hit: the wide BLAS trees cover the
 // same triangles with boxes that contain the reference boxes, and the device TLAS covers every
-// instance's geometry; only the visiting order (exact-t ties) can differ.
+// instance's geometry; only the visiting order (exact-t ties) can differ from the reference's.
 // ---------------------------------------------------------------------------------------
 struct Item {
   bool inner;       // inner binary node (else: primitive range)
@@ -609,6 +614,7 @@ struct Collapser {
   // memo: primitive range and leaf count of a subtree, one entry per binary node, sized by the
   // caller; collapsers of disjoint trees share it (each writes only its own nodes' entries)
   std::vector<Span>* span = nullptr;
+  bool leaves_pushed = false;  // the traversal pushes the leaf slots too (TLAS)
 
   // [first, end) of the primitives below binary node n.  bvh.rs partitions in place, so a
   // subtree covers a contiguous range (count == end - first); trees handed in through
@@ -785,14 +791,13 @@ struct Collapser {
   // builds the wide tree rooted at binary node `root`; returns the index of its root
   uint32_t build(uint32_t root) {
     dp_prepare(item_of(root));
-    std::vector<int32_t> queue{0};
-    size_t head = 0;
     const uint32_t base = (uint32_t)out->size();
+    std::vector<std::pair<int32_t, uint32_t>> queue{{0, base}};  // item, its node
+    size_t head = 0;
     out->push_back(WideNode{});
     std::vector<int32_t> items;
     while (head < queue.size()) {
-      const int32_t cur = queue[head];
-      const uint32_t self = base + (uint32_t)head;
+      const auto [cur, self] = queue[head];
       ++head;
       items.clear();
       if (dp[cur].l >= 0) {
@@ -802,25 +807,29 @@ struct Collapser {
       } else {
         items.push_back(cur);
       }
-      std::stable_partition(items.begin(), items.end(), [&](int32_t x) { return dp[x].l >= 0; });
+      auto is_inner = [&](int32_t x) { return dp[x].l >= 0; };
+      if (!leaves_pushed) std::stable_partition(items.begin(), items.end(), is_inner);
       WideNode w{};
       std::vector<Item> slots;
-      w.child_base = (uint32_t)out->size();
-      const uint32_t first_leaf = (uint32_t)(prim_order->size() / max_leaf);
-      uint32_t n_inner = 0;
-      for (const int32_t x : items) {
-        const Item& it = dp[x].it;
-        if (dp[x].l >= 0) {
-          ++n_inner;
-          queue.push_back(x);
-          out->push_back(WideNode{});
-        } else {
-          for (uint32_t i = 0; i < max_leaf; ++i) prim_order->push_back(i < it.count ? it.start + i : kNoPrim);
-        }
-        slots.push_back(it);
+      uint32_t inner = 0;
+      for (size_t k = 0; k < items.size(); ++k) {
+        inner |= (uint32_t)is_inner(items[k]) << k;
+        slots.push_back(dp[items[k]].it);
       }
-      w.leaf_base = first_leaf - n_inner;
-      w.set_children((uint32_t)slots.size(), n_inner);
+      w.set_children((uint32_t)slots.size(), inner);
+      const uint32_t leaves = w.bits & 0xFFu & ~inner;
+      // the records of slots first .. last of a kind; base is that of slot 0, modulo 2^32
+      auto first = [](uint32_t mask) { return mask ? (uint32_t)__builtin_ctz(mask) : 0u; };
+      w.child_base = (uint32_t)out->size() - first(inner);
+      w.leaf_base = (uint32_t)(prim_order->size() / max_leaf) - first(leaves);
+      for (size_t k = 0; k < items.size(); ++k) {
+        const Item& it = slots[k];
+        if (inner >> k & 1u) queue.push_back({items[k], w.child_base + (uint32_t)k});
+        if (inner >> k && k >= first(inner)) out->push_back(WideNode{});
+        if (!(leaves >> k) || k < first(leaves)) continue;
+        const uint32_t n = leaves >> k & 1u ? it.count : 0u;
+        for (uint32_t i = 0; i < max_leaf; ++i) prim_order->push_back(i < n ? it.start + i : kNoPrim);
+      }
       quantise(&w, slots);
       (*out)[self] = w;
     }
@@ -923,7 +932,7 @@ std::vector<TlasEntry> tlas_entries(const HostScene& s, const std::vector<uint32
   for (size_t i = 0; i < s.instances.size(); ++i) {
     const uint32_t root = s.wblas_root[inst_blas[i]];
     const WideNode& w = s.wblas[root];
-    bool split = w.n_children() > 1 && w.n_inner() == w.n_children();
+    bool split = w.n_children() > 1 && w.inner() == (w.bits & 0xFFu);
     if (split) {
       float ib[6];
       instance_box(s.instances[i], s.blas[s.instances[i].node], ib);
@@ -962,7 +971,7 @@ void entry_boxes(const HostScene& s, const std::vector<uint32_t>& tri_order, con
       const WideNode& w = s.wblas[st.back()];
       st.pop_back();
       for (uint32_t c = 0; c < w.n_children(); ++c) {
-        if (c < w.n_inner()) {
+        if (w.inner() >> c & 1u) {
           st.push_back(w.child_base + c);
           continue;
         }
@@ -1119,6 +1128,7 @@ int to_device_layout(HostScene* s) {
   s->wtlas.clear();
   s->itrace.clear();
   s->tlas_entries = 0;
+  s->wtlas_nodes = 0;
   s->ishade.assign(n_inst, GpuInstShade{});
   s->has_tlas = !s->tlas.empty() && n_inst > 0;
   if (s->has_tlas) {
@@ -1134,11 +1144,12 @@ int to_device_layout(HostScene* s) {
       for (int q = 0; q < 3; ++q) { ebox[6 * k + q] = eb[k].mn[q]; ebox[6 * k + 3 + q] = eb[k].mx[q]; }
     std::vector<uint32_t> order;
     std::vector<Collapser::Span> tmemo(tlas.size());
-    Collapser ct{tlas, ebox, &s->wtlas, &order, 1, &tmemo};
+    Collapser ct{tlas, ebox, &s->wtlas, &order, 1, &tmemo, true};
     ct.build(0);  // raytracing_sw.wgsl:183-186: the TLAS root is node 0
     s->itrace.assign(order.size(), GpuInstTrace{});
-    s->tlas_entries = order.size();
+    s->tlas_entries = eb.size();
     for (size_t k = 0; k < order.size(); ++k) {
+      if (order[k] == kNoPrim) continue;
       const TlasEntry& en = entries[eb[order[k]].payload];
       const nb_instance& in = s->instances[en.inst];
       GpuInstTrace& tr = s->itrace[k];
@@ -1148,6 +1159,7 @@ int to_device_layout(HostScene* s) {
       tr.ref_index = en.inst;
     }
   }
+  for (const WideNode& w : s->wtlas) s->wtlas_nodes += w.n_children() != 0;
   for (size_t i = 0; i < n_inst; ++i) {
     const nb_instance& in = s->instances[i];
     GpuInstShade& sh = s->ishade[i];
