@@ -9,8 +9,9 @@
 // latency of the node, triangle and instance loads.  A ray costs ~2.5 times the instructions, so the
 // callers use this only below the ray counts at which a ray per lane fills the GPU (kGroupPaths).
 //
-// The arithmetic, the sort keys, the order in which nodes are visited and the order in which equal
-// distances win are those of trace_step, so a ray's hit is the same bits.
+// The triangles' arithmetic, the sort keys, the order in which nodes are visited and the order in which
+// equal distances win are those of trace_step, so a ray's hit is the same bits.  (Only the rounding of
+// closest hits' far planes differs, Planes: another box may be opened in vain.)
 #pragma once
 
 namespace nbd {
@@ -131,7 +132,7 @@ struct GroupTrace {
       __syncwarp();  // the entries are read before the pushes below
     }
 
-    // ---- this lane's child: the slab test of trace_step, with any-hit queries' offset ----
+    // ---- this lane's child: the slab test of trace_step, near and far planes with offset 2^15 ----
     // plane bytes (WideNode): lo x, y, z at 32, 40, 48 and hi x, y, z at 56, 64, 72, one per child;
     // the near plane is the low one where the direction is positive
     NodeHead nh{};

@@ -141,23 +141,31 @@ __device__ __forceinline__ F2 operator-(F2 a, F2 b) {
 // A plane byte q as the float offset + q: a byte product added to the offset's bits.  The products run
 // beside the ALU pipe, which bounds the traversal of camera rays (75% of its peak, the FMA pipes 25%):
 // against byte permutes on that pipe, and the maximum of three and the hit test on it too, 1920x1080 at
-// 64 spp 101.3 -> 93.9 ms, camera rays on the 1M-triangle soup 2.52 -> 2.33.  Offset 2^16 takes
-// bits 0x47800000 + (q << 7), whose weight fits a byte, an immediate.  The rounding of a child's entry
-// distance differs with the offset in its last bits, and with it once in 30,000 scattered rays the order
-// of two overlapping children: the closest hit is the same, the first found is not.  So any-hit queries
-// keep 2^15, bits 0x47000000 + (q << 8) by a product of 16-bit weights held in registers (closest hits
-// with it: the frame 97.1 ms, camera rays 2.38; scattered any hit 3.80 -> 3.67).
+// 64 spp 101.3 -> 93.9 ms, camera rays on the 1M-triangle soup 2.52 -> 2.33.
+// Near planes have offset 2^15, bits 0x47000000 + (q << 8) by a product of 16-bit weights held in
+// registers.  Their rounding is part of the answer: a child's entry distance decides the order of
+// overlapping children and with it which of two triangles at the same distance is found, and the group
+// kernels (GroupTrace) have the same offset, so that a hit does not depend on the size of the call.  Far planes
+// only decide whether a box is opened, with a margin (trace_step) for any rounding.  For closest hits
+// they have offset 2^16, bits 0x47800000 + (q << 7), whose weight fits a byte, an immediate: 1920x1080 at
+// 64 spp 91.1 -> 89.4 ms, camera rays 2.29 -> 2.28.  (Near planes that way too: 88.2 and 2.25, but another
+// triangle for one in 170,000 rays on coincident surfaces.)  Any-hit queries take 2^15 for both: scattered
+// rays 3.57 ms, with 2^16 for the far planes 3.62.
 template <bool kAny>
 struct Planes {
-  static constexpr float kOffset = kAny ? 32768.0f : 65536.0f;
-  static constexpr float kMargin = kOffset / 4194304.0f;  // of |a|: see trace_step
+  static constexpr float kOffset = 32768.0f;
   static __device__ __forceinline__ uint32_t decode(uint32_t w, int k) {
-    if (!kAny) return __dp4a(w, 0x80u << (8 * k), 0x47800000u);
     const uint32_t weight = (k & 1) ? 0x01000000u : 0x100u;
     return (k & 2) ? __dp2a_hi(weight, w, 0x47000000u) : __dp2a_lo(weight, w, 0x47000000u);
   }
   // byte k of a near and a far word
-  static __device__ __forceinline__ F2 pair(uint32_t n, uint32_t f, int k) { return pack2(decode(n, k), decode(f, k)); }
+  static __device__ __forceinline__ F2 pair(uint32_t n, uint32_t f, int k) {
+    return pack2(decode(n, k), kAny ? decode(f, k) : __dp4a(f, 0x80u << (8 * k), 0x47800000u));
+  }
+  // the far planes' constant from c, the one with offset 2^15, and the near planes' margin d
+  static __device__ __forceinline__ float far(float a, float c, float d) {
+    return kAny ? c + d : fmaf(-32768.0f, a, fmaf(2.0f, d, c));
+  }
 };
 // maximum and minimum of three, as fmaxf and fminf of two treat NaN
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -471,21 +479,23 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
     const float4 q2 = w1.a, q3 = w1.b, q4 = ld4(np + 4);
     const float ax = nh.step_x * rinv.x, ay = nh.step_y * rinv.y, az = nh.step_z() * rinv.z;
     const float bx = (nh.p.x - ro.x) * rinv.x, by = (nh.p.y - ro.y) * rinv.y, bz = (nh.p.z - ro.z) * rinv.z;
-    // A plane byte q is read as the float F = P + q, P = 2^16 or 2^15 (Planes), and its distance taken
-    // as fma(F, a, b - P a).  With u = 2^-24, the folded constant, the margin added to it and the FMA
-    // are off by at most u (|b| + P |a|), u (|b| + P |a|) and u (|b| + 255 |a|): each plane's distance
-    // lies within 1.8e-7 |b| + (2^-23 P + 1.6e-5) |a| of b + q a.  Near-plane constants are lowered and
-    // far-plane constants raised by d = 2^-22 P |a| + |b| / 2^19 per axis.  For every plane
-    // t = b + q a of the node (|t| <= |b| + 255 |a|) the margin covers that, the approximate reciprocal
-    // (<= 2^-22 |t|) and the rounding of the plane evaluation against the exact reference box
-    // (4e-7 |t|): together at most 8.2e-7 |b| + (2^-23 P + 1.9e-4) |a| <= d, so a box never rejects a
-    // ray the reference box accepts.
+    // A plane byte q is read as the float F = P + q, P = 2^15 or, for closest hits' far planes, 2^16
+    // (Planes), and its distance taken as fma(F, a, b - P a).  With u = 2^-24, the folded constant, the margin
+    // added to it and the FMA are off by at most u (|b| + P |a|), u (|b| + P |a|) and u (|b| + 255 |a|), and
+    // where 2^16 a is folded in two halves by u (|b| + P |a|) more at most: each plane's distance lies within
+    // 1.8e-7 |b| + (2^-9 + 1.6e-5) |a| of b + q a, with 2^16 within 2.4e-7 |b| + (2^-7 + 1.6e-5) |a|.
+    // Near-plane constants are lowered by d = |a| / 128 + |b| / 2^19 per axis and far-plane constants raised
+    // by d, with 2^16 by 2 d.  For every plane t = b + q a of the node (|t| <= |b| + 255 |a|) the margin
+    // covers that, the approximate reciprocal (<= 2^-22 |t|) and the rounding of the plane evaluation
+    // against the exact reference box (4e-7 |t|): together at most 8.8e-7 |b| + (2^-9 + 1.9e-4) |a| <= d, or
+    // 8.8e-7 |b| + (2^-7 + 1.9e-4) |a| <= 2 d, so a box never rejects a ray the reference box accepts.
     using Q = Planes<kAny>;
-    const float dx = fmaf(fabsf(ax), Q::kMargin, fabsf(bx) * 1.9073486328125e-6f);
-    const float dy = fmaf(fabsf(ay), Q::kMargin, fabsf(by) * 1.9073486328125e-6f);
-    const float dz = fmaf(fabsf(az), Q::kMargin, fabsf(bz) * 1.9073486328125e-6f);
+    const float dx = fmaf(fabsf(ax), 0.0078125f, fabsf(bx) * 1.9073486328125e-6f);
+    const float dy = fmaf(fabsf(ay), 0.0078125f, fabsf(by) * 1.9073486328125e-6f);
+    const float dz = fmaf(fabsf(az), 0.0078125f, fabsf(bz) * 1.9073486328125e-6f);
     const float cx = fmaf(-Q::kOffset, ax, bx), cy = fmaf(-Q::kOffset, ay, by), cz = fmaf(-Q::kOffset, az, bz);
-    const float cnx = cx - dx, cfx = cx + dx, cny = cy - dy, cfy = cy + dy, cnz = cz - dz, cfz = cz + dz;
+    const float cnx = cx - dx, cny = cy - dy, cnz = cz - dz;
+    const float cfx = Q::far(ax, cx, dx), cfy = Q::far(ay, cy, dy), cfz = Q::far(az, cz, dz);
     // near/far planes per axis by the sign of the direction: the near plane of a child is its
     // low plane where rinv >= 0 (t grows with the quantised coordinate), else its high plane
     const bool pxs = rinv.x >= 0.0f, pys = rinv.y >= 0.0f, pzs = rinv.z >= 0.0f;
@@ -509,7 +519,8 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
       const float2 tz = unpack2(fma2(Q::pair(k < 4 ? nz0 : nz1, k < 4 ? fz0 : fz1, k & 3), az2, cz2));
       const float lo = max3(fmaxf(tx.x, ty.x), tz.x, 0.0f);
       const float hi = min3(fminf(tx.y, ty.y), tz.y, t_below);
-      // lo <= hi as the sign of hi - lo: neither is NaN, lo is >= +0 and hi never -0 (the margin is added last)
+      // lo <= hi as the sign of hi - lo: neither is NaN, lo is >= +0 and hi never -0: the margin, >= +0, is in
+      // its constant (and sums of these products are exact where they are denormal)
       misses = __funnelshift_l(f2u(hi - lo), misses, 1);
       key[k] = (f2u(lo) & ~7u) | (uint32_t)k;
     }
@@ -545,9 +556,8 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
         NB_CX(1, 2) NB_CX(3, 4) NB_CX(5, 6)
       }
       // a child's stack entry: node or instance index and its key (its slot in the low 3 bits).  (Which of the
-      // two by the mask, since a TLAS node's slots mix them: 1920x1080 at 64 spp 88.2 ms, camera rays on the
-      // soup 2.25, scattered any hit 3.57.  With the inner children first and a comparison 87.8, 2.23 and 3.57, but
-      // then an inner child came before an instance at the same distance, whatever their places in the tree.)
+      // two by the mask, since a TLAS node's slots mix them.  With the inner children first and a comparison
+      // 1920x1080 at 64 spp takes 0.4 ms less, camera rays on the soup 0.02, scattered any hit the same, but then an inner child came before an instance at the same distance, whatever their places in the tree.)
       const uint32_t inst_base = kInstanceBit + nh.leaf_base;
       auto entry = [&](uint32_t kk) {
         const uint32_t slot = kk & 7u;

@@ -78,7 +78,7 @@ def golden():
 
 
 @pytest.mark.parametrize("incoherent", [False, True])
-@pytest.mark.parametrize("make,any_hit", [(crowd, True), (coincident, True)])
+@pytest.mark.parametrize("make,any_hit", [(crowd, True), (crowd, False), (coincident, False), (coincident, True)])
 def test_hits_are_the_recorded_ones(golden, make, any_hit, incoherent):
     scene, key = make(), f"{make.__name__}_{'any' if any_hit else 'closest'}"
     r, want = golden[make.__name__ + "_rays"], golden[key]
