@@ -1868,12 +1868,24 @@ int nb_cache_infer(nb_cache* c, const float* enc, size_t n, float* out, void* st
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int sms = sm_count();
+  // The rows are read while earlier ones' outputs are written: outputs that lie in the rows' memory go
+  // through the scratch buffer.
+  const uintptr_t in0 = reinterpret_cast<uintptr_t>(enc), out0 = reinterpret_cast<uintptr_t>(out);
+  const size_t out_bytes = n * 3 * sizeof(float);
+  const bool overlap = out0 < in0 + n * 64 * sizeof(float) && in0 < out0 + out_bytes;
   if (c->cfg.tensor_path == NB_CACHE_TCGEN05) {
+    float* dst = out;
+    if (overlap) {
+      if ((rc = ensure_scratch(c, n))) return rc;
+      dst = reinterpret_cast<float*>(c->sx);
+    }
     c->report->status = 0;
     const size_t groups = (n + nbd::kTcRows - 1) / nbd::kTcRows;
     nbd::k_cache_infer_tc<false><<<(unsigned)std::min<size_t>(groups, (size_t)sms), nbd::kTcThreads,
-                                   nbd::kTcSmem, st>>>(c->wb, enc, nullptr, nullptr, (uint32_t)n, c->bounds, out,
+                                   nbd::kTcSmem, st>>>(c->wb, enc, nullptr, nullptr, (uint32_t)n, c->bounds, dst,
                                                        nullptr, nullptr, &c->report->status);
+    NB_CUDA(cudaGetLastError(), "cache infer launch");
+    if (overlap) NB_CUDA(cudaMemcpyAsync(out, dst, out_bytes, cudaMemcpyDeviceToDevice, st), "cudaMemcpyAsync");
   } else {
     if ((rc = ensure_scratch(c, n))) return rc;
     nbd::k_to_bf16<<<grid_for(n * 64, 256, sms), 256, 0, st>>>(enc, c->sx, n * 64);
