@@ -687,7 +687,7 @@ static int render_samples(nb_pathtracer* pt, const nb_scene* scene, const nb_cam
       if (rc) return rc;
       if (e == cudaSuccess)
         e = timed_launch(pt, kKindCacheTrain, st, [&] {
-          rc = cache_wave_train(pt->cache, wt.n_paths, pt->sms, st);
+          rc = cache_wave_train(pt->cache, pb, wt.n_paths, pt->sms, st);
           return cudaSuccess;
         });
       if (rc) return rc;

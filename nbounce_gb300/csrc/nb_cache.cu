@@ -1402,9 +1402,11 @@ struct nb_cache {
   nbd::bf16* web = nullptr;
   float* m = nullptr;
   float* v = nullptr;
-  // Tensor-core wait timeouts of nb_cache_infer / training, and the loss of a caller's batch: in
+  // Tensor-core wait timeouts and the loss of a caller's batch (nb_cache_infer, _gradient, _train_step): in
   // page-locked host memory that the kernels write (the status only on a timeout), so that a call
-  // that reports them needs a stream synchronisation and no copies
+  // that reports them needs a stream synchronisation and no copies.  The host clears the status, so
+  // only kernels that the same call waits for may have it; a wave's lookups and training, which stay in
+  // flight, raise theirs in the wave's device status word
   struct Report {
     uint32_t status;
     float loss;
@@ -1550,14 +1552,15 @@ int grid_for(size_t n, int threads, int sms) {
 
 // one optimiser step (update) or gradient evaluation over rows [row0, row0 + rows_per_step)
 // of (X, Y); n_dev (device row count) or n_host bounds the rows
-// raw: X and Y are the caller's FP32 rows and targets (tcgen05 path only)
+// raw: X and Y are the caller's FP32 rows and targets (tcgen05 path only).  status takes the tensor-core
+// waits that gave up: the word of the call or wave whose rows these are, never another's.
 cudaError_t train_launch(nb_cache* c, const void* X, const void* Y, bool raw, const uint32_t* n_dev, uint32_t n_host,
                          uint32_t row0, uint32_t rows_per_step, bool update, float* grad_out, float* loss_out,
-                         cudaStream_t st) {
+                         uint32_t* status, cudaStream_t st) {
   const uint32_t ctas = (rows_per_step + nbd::kGradRows - 1) / nbd::kGradRows;
   if (c->cfg.tensor_path == NB_CACHE_TCGEN05)
     (raw ? nbd::k_cache_grad_tc<true> : nbd::k_cache_grad_tc<false>)<<<ctas, 128, nbd::kTrSmem, st>>>(
-        c->wstage, X, Y, n_dev, n_host, row0, rows_per_step, c->cfg.grad_clip, c->part_dw, c->part_loss, &c->report->status);
+        c->wstage, X, Y, n_dev, n_host, row0, rows_per_step, c->cfg.grad_clip, c->part_dw, c->part_loss, status);
   else
     nbd::k_cache_grad<<<ctas, 256, nbd::kGradSmem, st>>>(c->wb, static_cast<const nbd::bf16*>(X),
                                                          static_cast<const float4*>(Y), n_dev, n_host, row0,
@@ -1696,7 +1699,7 @@ int cache_wave_infer(nb_cache* c, const PathBatch& pb, int sms, cudaStream_t st)
 }
 
 // Then: training records from the training paths' chains and the optimiser steps.
-int cache_wave_train(nb_cache* c, uint32_t n_paths, int sms, cudaStream_t st) {
+int cache_wave_train(nb_cache* c, const PathBatch& pb, uint32_t n_paths, int sms, cudaStream_t st) {
   const uint32_t tiles = (c->cap_slots + nbd::kScanTile - 1) / nbd::kScanTile;
   nbd::k_cache_count<<<tiles, nbd::kScanThreads, 0, st>>>(c->vert_count, c->cap_slots, n_paths, c->stride,
                                                           c->block_sums, c->counters);
@@ -1716,7 +1719,7 @@ int cache_wave_train(nb_cache* c, uint32_t n_paths, int sms, cudaStream_t st) {
   const uint32_t per = steps ? (c->cfg.train_records + steps - 1) / steps : 0;
   for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k)
     e = train_launch(c, c->X, c->Y, false, c->counters + 2, 0, k * per, per, c->cfg.learning_rate > 0.0f, nullptr,
-                     c->losses + k, st);
+                     c->losses + k, pb.status, st);
   if (e != cudaSuccess) return cuda_fail(e, "cache wave launch");
   c->last_steps = steps;
   c->frame += 1;
@@ -1924,7 +1927,7 @@ static int rows_op(nb_cache* c, const float* enc, const float* target, size_t n,
   }
   if (e == cudaSuccess)
     e = train_launch(c, tc ? (const void*)enc : c->sx, tc ? (const void*)target : c->sy, tc, nullptr, (uint32_t)n, 0,
-                     (uint32_t)n, update, grad, &c->report->loss, st);
+                     (uint32_t)n, update, grad, &c->report->loss, &c->report->status, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "cache training launch");
   if (loss) *loss = *(volatile float*)&c->report->loss;

@@ -120,5 +120,5 @@ int cache_wave_begin(nb_cache* c, const nb_scene* scene, uint32_t n_paths, Cache
 // after the last bounce: cache lookups (image queries and training-path tails)
 int cache_wave_infer(nb_cache* c, const PathBatch& pb, int sms, cudaStream_t st);
 // then: training records and optimiser steps
-int cache_wave_train(nb_cache* c, uint32_t n_paths, int sms, cudaStream_t st);
+int cache_wave_train(nb_cache* c, const PathBatch& pb, uint32_t n_paths, int sms, cudaStream_t st);
 }  // namespace nb

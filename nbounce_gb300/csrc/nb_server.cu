@@ -358,7 +358,7 @@ struct nb_server {
     cudaError_t e = launch_bounces(p, *wt, Estimator::kCache, true, max_bounces, sq, cw, d_rays, sms, stream,
                                    group_wave(), nullptr, [](Stage, auto launch) { return launch(); });
     if (e != cudaSuccess) return cuda_fail(e, "cache wave launch");
-    if ((rc = cache_wave_infer(c, p, sms, stream)) || (rc = cache_wave_train(c, wt->n_paths, sms, stream)))
+    if ((rc = cache_wave_infer(c, p, sms, stream)) || (rc = cache_wave_train(c, p, wt->n_paths, sms, stream)))
       return rc;
     e = launch_accumulate(p, *wt, sms, stream);
     return e == cudaSuccess ? NB_OK : cuda_fail(e, "cache wave launch");
