@@ -598,27 +598,14 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
     }
 #undef NB_CX
   }
-  if (kCount) {
-    const uint32_t together = __activemask();
-    uint32_t n_tris = 0;
-    if (leaf_mask) {
-      const uint32_t k = (uint32_t)(__ffs(leaf_mask) - 1);
-      n_tris = f2u(ld4(s.tris + 6 * (size_t)(t.leaf_base + k) + 4).w) == 0xFFFFFFFFu ? 1u : 2u;
-    }
-    cnt->tris += n_tris;
-    const uint32_t with_leaves = __ballot_sync(together, leaf_mask != 0u);
-    const uint32_t most = __reduce_max_sync(together, n_tris);
-    if (with_leaves && lowest_active(together)) {
-      ++cnt->leaf_steps;
-      cnt->leaf_lanes += (uint32_t)__popc(with_leaves);
-      cnt->leaf_trips += most;
-    }
-  }
+  uint32_t together = 0, n_tris = 0;  // kCount: the lanes of this step, triangles tested by this one
+  if (kCount) together = __activemask();
   // ---- BLAS leaf slots: Moller-Trumbore (raytracing_sw.wgsl:51-78, 274-286), all of the node's or as
   // many as enough lanes have (kLeafLanes) ----
   while (leaf_mask) {
     const uint32_t k = (uint32_t)(__ffs(leaf_mask) - 1);
     leaf_mask &= leaf_mask - 1;
+    if (kCount) n_tris += f2u(ld4(s.tris + 6 * (size_t)(t.leaf_base + k) + 4).w) == 0xFFFFFFFFu ? 1u : 2u;
     bool found = false;
     triangle_pair_test(ro, rd, s.tris + 6 * (size_t)(t.leaf_base + k), h_t,
                        [&](float t, float u, float v, uint32_t tri) {
@@ -630,6 +617,17 @@ __device__ __forceinline__ bool trace_step(TraceState& t, const Stack& stack, co
                        });
     if (kAny && found) return false;
     if (Stack::kScattered && __popc(__ballot_sync(__activemask(), leaf_mask != 0u)) < kLeafLanes) break;
+  }
+  if (kCount) {  // closest hits only: every lane of the step comes here
+    static_assert(!(kCount && kAny), "a lane whose any-hit query ends leaves the step");
+    cnt->tris += n_tris;
+    const uint32_t with_leaves = __ballot_sync(together, n_tris != 0u);
+    const uint32_t most = __reduce_max_sync(together, n_tris);
+    if (with_leaves && lowest_active(together)) {
+      ++cnt->leaf_steps;
+      cnt->leaf_lanes += (uint32_t)__popc(with_leaves);
+      cnt->leaf_trips += most;
+    }
   }
   return true;
 }
