@@ -7,6 +7,8 @@
 #pragma once
 
 #include <cstdint>
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include "nb_device.cuh"
@@ -122,15 +124,18 @@ enum class Estimator { kPlain, kNee, kCache };
 cudaError_t launch_trace_paths(const PathBatch& pb, const WaveTables& wt, Estimator est, const CacheWave& cw,
                                uint32_t bounce, unsigned long long* ray_total, int sms, cudaStream_t st);
 
-// Queues and waves up to kGroupPaths paths, and nb_trace_rays calls up to kGroupRays rays
-// (kGroupScattered with NB_TRACE_INCOHERENT), are traced by 8 lanes per ray.  Such a ray costs ~2.5 times the instructions of a ray per lane, but a node step
-// takes 0.8 us instead of ~2, and a launch is as long as its longest ray until the GPU is full.
+// Queues and waves up to kGroupPaths paths (fewer where they can have few more rays or have shadow rays:
+// launch_bounces), and nb_trace_rays calls up to kGroupRays rays (kGroupScattered with
+// NB_TRACE_INCOHERENT), are traced by 8 lanes per ray.  Such a ray costs ~2.5 times the instructions of a
+// ray per lane, but a node step takes 0.8 us instead of ~2, and a launch is as long as its longest ray
+// until the GPU is full.
 // Paths (run to their ends by k_trace_paths), limits of 16K / 24K / 32K / 64K: 160x120 at 1 spp on the
 // instanced scene 320 / 260 / 262 / 260 us, 256x256 514 / 516 / 517 / 642, with NEE 1000 / 1000 / 1194 /
 // 1544, 400x300 626 / 631 / 594 / 679, 576x320 669 / 657 / 653 / 642, 1013x571 at 3 spp with NEE 3025 / 3090 /
-// 3080 / 3348.  Rays, 8 lanes against one, closest hits: camera grids of 16,384 rays on soups of 2K, 20K and
-// 1M triangles 24 / 24, 50 / 58 and 108 / 145 us, of 32,761 rays 33 / 23, 63 / 59 and 156 / 178; 24,025
-// scattered rays 37 / 38, 76 / 92 and 190 / 250, 32,761 44 / 40, 91 / 94 and 218 / 256.
+// 3080 / 3348 (queues handed on whatever their length from some bounce on, which is no longer done).  Rays, 8
+// lanes against one, closest hits: camera grids of 16,384 rays on soups of 2K, 20K and 1M triangles 24 / 24,
+// 50 / 58 and 108 / 145 us, of 32,761 rays 33 / 23, 63 / 59 and 156 / 178; 24,025 scattered rays 37 / 38,
+// 76 / 92 and 190 / 250, 32,761 44 / 40, 91 / 94 and 218 / 256.
 constexpr uint32_t kGroupPaths = 1u << 15;
 constexpr uint32_t kGroupRays = 1u << 14, kGroupScattered = 3u << 13;
 
@@ -145,18 +150,34 @@ cudaError_t launch_bounces(const PathBatch& pb, WaveTables& wt, Estimator est, b
                            const ShadowQueue& sq, const CacheWave& cw, unsigned long long* ray_total, int sms,
                            cudaStream_t st, bool groups, unsigned long long* counters, Timed timed) {
   groups = groups && counters == nullptr;
-  wt.group_limit = groups ? kGroupPaths : 0u;
+  wt.group_limit = 0u;
   wt.flags = est != Estimator::kPlain ? kWaveZeroRadiance : 0u;  // their shading adds to radiance
-  // From bounce `last` on every queue goes to k_trace_paths, whatever its length, and the launches of
-  // later bounces are saved: there the queue holds at most kGroupPaths paths if half of the paths end
-  // per bounce (half to two thirds do in open scenes; where most survive, both ways took the same time
-  // within 10%).
-  uint32_t last = 0;
-  while (groups && (wt.n_paths >> last) > kGroupPaths) ++last;
+  // Whether a bounce's queue is short (limit) is decided on the device, at each bounce up to the one after
+  // that where it is short if half of the paths end per bounce, and at every second one after it: as many
+  // of open scenes' queues as ever get short have done so by then, and a check that finds nothing to do, or a
+  // bounce whose paths have ended, costs 3 to 4 us a launch.  How many paths a bounce leaves is the
+  // scene's: handing every queue to k_trace_paths from that bounce on, whatever its length, saves those
+  // launches (576x320 at 1 spp on the instanced scene 662 instead of 731 us), but an enclosed scene keeps
+  // most of its paths alive.  The room (scenes.room_scene), with / without that rule: 576x320 at
+  // 1 spp 1013 / 583 us, 1920x1080 4186 / 2276, at 12 bounces 5365 / 2575, 256x256 at 16 spp 3474 / 1462, 1920x1080
+  // with NEE 8234 / 3318.  Checks at every bounce: 2,000 overlapping spheres at 576x320 11.6 instead of 11.0 ms,
+  // the instanced scene 733 us; none after the first kind: 14.1 instead of 12.2 at 12 bounces, 713 us.
+  //
+  // A path that can have few more rays gains little from a launch of its own to its end, and an enclosed
+  // scene's paths have all they can.  181x181 pixels of the room at 0 / 1 / 2 / 3 / 4 / 6 bounces: per bounce 60 / 121 /
+  // 174 / 221 / 269 / 360 us, as one launch 90 / 174 / 241 / 298 / 337 / 402; 150x150 at 0 to 4: 62 / 115 / 165 / 212 / 261
+  // and 68 / 126 / 174 / 216 / 244.  With NEE, whose shadow rays share the per-bounce launches, 181x181 at 3 / 6
+  // bounces 297 / 469 and 651 / 886 us; 1013x571 at 3 spp of the instanced scene takes 2.98 ms, 3.05 with a limit
+  // of 32,768.
+  const uint32_t cap = est == Estimator::kNee ? 3u * (kGroupPaths / 4u) : kGroupPaths;
+  auto limit = [&](uint32_t b) { return std::min(cap, 4096u * (max_bounces + 2u - b)); };
+  uint32_t half = 0;
+  while (groups && half <= max_bounces && (wt.n_paths >> half) > limit(half)) ++half;
+  auto check = [&](uint32_t b) { return groups && b >= 1 && (b <= half + 1 || ((b - half) & 1u)); };
   auto paths = [&](uint32_t b) {
     return timed(Stage::kTrace, [&] { return launch_trace_paths(pb, wt, est, cw, b, ray_total, sms, st); });
   };
-  if (groups && last == 0) {
+  if (groups && half == 0) {
     bool direct = est != Estimator::kCache;
     for (uint32_t k = 0; k < wt.n_segs; ++k) direct = direct && wt.segs[k].n_samples == 1;
     wt.flags = direct ? kWaveDirect : 0u;
@@ -172,14 +193,11 @@ cudaError_t launch_bounces(const PathBatch& pb, WaveTables& wt, Estimator est, b
     return timed(Stage::kTrace, [&] { return launch_trace_shadow(pb, wt, sq, b, sms, st); });
   };
   for (uint32_t b = 0; b <= max_bounces && e == cudaSuccess; ++b) {
-    const bool to_end = groups && b == last;
-    if (groups) wt.group_limit = to_end ? 0xFFFFFFFFu : kGroupPaths;
-    if (!to_end || mixed)
-      e = timed(Stage::kTrace, [&] {
-        return launch_trace_wave(pb, wt, single_scene, b, mixed ? &sq : nullptr, ray_total, sms, st, counters);
-      });
-    if (e == cudaSuccess && groups && b >= 1) e = paths(b);  // after the shadow rays: it goes on from their sums
-    if (to_end) return e;
+    wt.group_limit = check(b) ? limit(b) : 0u;
+    e = timed(Stage::kTrace, [&] {
+      return launch_trace_wave(pb, wt, single_scene, b, mixed ? &sq : nullptr, ray_total, sms, st, counters);
+    });
+    if (e == cudaSuccess && check(b)) e = paths(b);  // after the shadow rays: it goes on from their sums
     if (e == cudaSuccess)
       e = timed(Stage::kShade, [&] {
         return est == Estimator::kCache ? launch_shade_cache(pb, wt, cw, b, sms, st)
