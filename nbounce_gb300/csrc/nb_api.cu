@@ -692,7 +692,8 @@ static int render_samples(nb_pathtracer* pt, const nb_scene* scene, const nb_cam
         });
       if (rc) return rc;
     }
-    if (e == cudaSuccess) e = timed_launch(pt, kKindAccumulate, st, [&] { return launch_accumulate(pb, wt, pt->sms, st); });
+    if (e == cudaSuccess && !(wt.flags & kWaveDirect))
+      e = timed_launch(pt, kKindAccumulate, st, [&] { return launch_accumulate(pb, wt, pt->sms, st); });
     if (e != cudaSuccess) return cuda_fail(e, "path batch launch");
     pt->globals.sample += S;
     pt->globals.weight = 1.0f / (float)pt->globals.sample;
