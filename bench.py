@@ -49,17 +49,18 @@ if ROOT not in sys.path:
 
 METRIC = "Mrays/s (primary + extension rays), 1920x1080 64spp 8 bounces"
 # DRAM bytes (read + write) per traversal query of k_trace_wave over all bounces of a frame,
-# from one ncu capture of the same scene at 480x270, 64 spp (14 launches, 12,435,256 rays,
-# 915.4 MB read + 450.4 MB written); the roofline scales it to a launch by the launch's rays
-TRACE_DRAM_BYTES_PER_RAY = 109.8
+# from one ncu capture of the same scene at 480x270, 64 spp (17 launches, 12,435,256 rays,
+# 924.9 MB read + 449.5 MB written); the roofline scales it to a launch by the launch's rays
+TRACE_DRAM_BYTES_PER_RAY = 110.5
 # issue utilisation of the same capture (smsp__issue_active.avg.pct_of_peak_sustained_active):
 # camera rays (k_trace_wave<1,0,0>) and bounce 1 (the lane-refill kernel)
-TRACE_ISSUE_ACTIVE_PCT = {"camera_rays": 71.6, "bounce_1": 73.0}
+TRACE_ISSUE_ACTIVE_PCT = {"camera_rays": 70.9, "bounce_1": 72.8}
 UNIT = "Mrays/s"
 WORKLOAD = "instanced 16 meshes / 1024 instances, 1920x1080, 64 spp, 8 bounces, equirect sky"
 # bytes the device layout fetches per unit of traversal work (nb_trace_counters): an 8-wide
-# node, a triangle (half of a leaf slot's 80 bytes), an instance record, a stack entry written and read back; plus the
-# ray read from the queue (two float4) and the hit written (float4 + instance id)
+# node, a triangle (half of a leaf slot's 80 bytes; a slot of one triangle loads them all), an
+# instance record, a stack entry written and read back; plus the ray read from the queue (two
+# float4) and the hit written (float4 + instance id)
 NODE_BYTES, TRI_BYTES, INST_BYTES, PUSH_BYTES, RAY_IO_BYTES = 80, 40, 64, 16, 52
 TRUTH_DIR = os.path.join(ROOT, "tests", "golden")
 
@@ -676,7 +677,7 @@ def trace_roofline(pt, scene, cam, env, desc, kt, steps, rays_per_step, sh, of):
             "issue_active_pct": TRACE_ISSUE_ACTIVE_PCT,
             "note": "achieved = bytes the 8-wide device layout fetches (instrumented counters of one extra "
                     "frame) / timed trace launch time, against the HBM copy peak; mostly L1/L2 hits.  The "
-                    "binding limit is instruction issue (issue_active_pct: the schedulers issue in 72-73% of "
+                    "binding limit is instruction issue (issue_active_pct: the schedulers issue in 71-73% of "
                     "cycles, ncu on the 480x270 64-spp case) with SIMT divergence, not DRAM bandwidth"}
     if of is not None:
         n_aabb, n_tri, n_inst = of.work_per_ray()

@@ -11,7 +11,7 @@
 // memory as 336 rows x 64 inputs, rows padded to 72 elements so that ldmatrix is
 // conflict-free):
 //   k_cache_infer_tc tcgen05.mma (5th-generation tensor cores): weights in shared memory,
-//                    activations and FP32 accumulators in tensor memory, 8 groups of 128 rows per CTA
+//                    activations and FP32 accumulators in tensor memory, 4 groups of 128 rows per CTA
 //   k_cache_infer_*  mma.sync: one warp evaluates 32 rows, the activations never leave
 //                    registers (the C fragment of layer l, ReLU'd and packed to BF16, is the A
 //                    fragment of layer l + 1)
@@ -307,10 +307,10 @@ __global__ void __launch_bounds__(256, 2) k_cache_infer_queries(const bf16* __re
 // The warpgroup's first thread issues four K = 16 MMAs and commits them to the warpgroup's mbarrier;
 // then the warps read their accumulator rows (tcgen05.ld), apply ReLU, round to BF16 and store the
 // next layer's A (tcgen05.st).  Activations never pass through shared memory: with the operand there
-// (8 chains per SM) its stores and the MMAs' reads of it took 51% of the shared-memory pipe, all
-// requests 65%, and a million rows 101 us; this way they take 74 us (the rows' bytes 38 us, the
-// rest the latency of the chains: an MMA round trip, two barriers, the accumulator's load and the
-// operand's store per layer).  The caller's rows are loaded one group ahead, behind the
+// (8 chains per SM) the L1 and shared-memory unit ran at 65% of its peak and a million rows took 100 us;
+// this way it runs at 52% and they take 77 us (cold, under ncu; the rows' bytes 38 us, the rest the
+// latency of the chains: an MMA round trip, two barriers, the accumulator's load and the operand's store
+// per layer).  The caller's rows are loaded one group ahead, behind the
 // layers of the group before.  The warp-collective (.sync.aligned) tcgen05 instructions run on whole
 // converged warps.  Waits poll the mbarrier a bounded number of times: on a timeout the warpgroup
 // raises kStatusCacheTimeout (bits 16.. = 1 + the layer it waited for) and stops; the CTA frees its

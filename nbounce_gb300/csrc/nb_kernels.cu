@@ -285,12 +285,12 @@ constexpr int kWorldFloats = 9 * 32;
 constexpr int kTraceWarps = 4;  // every traversal kernel runs blocks of 128 threads
 constexpr int kTraceThreads = 32 * kTraceWarps;
 // Blocks per SM of the traversal kernels: with lane refill 7 (72 registers), whole-warp chunks 6 (80), of
-// closest-hit queries 7.  Camera grids of 2048x2048 with 6 / 7: closest hits on soups of 1M, 200K and 20K
+// closest-hit queries 7 (kQueryBlocks).  Camera grids of 2048x2048 with 6 / 7: closest hits on soups of 1M, 200K and 20K
 // triangles 2.28 / 2.23, 2.07 / 2.03 and 0.72 / 0.71 ms, on the instanced scene 1.35 / 1.32; any hits
 // 2.02 / 2.03, 2.04 / 2.06, 0.74 / 0.75 and 1.11 / 1.14, and a render's camera rays with 7 no faster than with
 // 6.  1920x1080 at 64 spp and scattered any hit, refill and chunk blocks 8+7: 103.5 and 4.79 ms, 7+6: 90.9
 // and 3.59, 6+5: 94.4 and 3.77.
-constexpr int kRefillBlocks = 7, kChunkBlocks = 6;
+constexpr int kRefillBlocks = 7, kChunkBlocks = 6, kQueryBlocks = 7;
 struct WorldRegs {
   const TraceState& t;
   __device__ __forceinline__ V3 o() const { return t.wo; }
@@ -389,8 +389,8 @@ __device__ __forceinline__ bool lowest_active(uint32_t mask) {
   return (threadIdx.x & 31u) == (uint32_t)(__ffs(mask) - 1);
 }
 
-// Bound by instruction issue, latency and divergence: the schedulers issue in 72% of cycles for camera rays
-// (ALU pipe 60% of its peak, 20 of 32 lanes active) and 73% for secondary rays (56%, 16 of 32; the
+// Bound by instruction issue, latency and divergence: the schedulers issue in 71% of cycles for camera rays
+// (ALU pipe 59% of its peak, 20 of 32 lanes active) and 73% for secondary rays (55%, 16 of 32; the
 // benchmark scene at 480x270, 64 spp).  Run twice, the leaf tests
 // add 16% to the 1080p frame (51% to scattered rays in the soup), the sort 4%, the pushes 2%.  What it costs per warp
 // step is its instructions, most of them not in the box tests: a slot's triangles are tested two at a
@@ -718,7 +718,7 @@ namespace nbd {
 // kRefill: lanes refill as they finish (trace_refill), for rays whose neighbours in the array
 // are unrelated; else each warp traces 32 consecutive rays to the end.
 template <bool kAny, bool kRefill>
-__global__ void __launch_bounds__(kTraceThreads, kRefill || !kAny ? kRefillBlocks : kChunkBlocks)
+__global__ void __launch_bounds__(kTraceThreads, kRefill ? kRefillBlocks : kAny ? kChunkBlocks : kQueryBlocks)
     k_trace_rays(DevScene s, const float4* __restrict__ rays, uint32_t n, float4* __restrict__ hits,
                  uint32_t* __restrict__ inst, uint32_t* __restrict__ fetch, uint32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
@@ -1950,7 +1950,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRefillBlocks) k_trace_shadow(P
   for (uint32_t i = threadIdx.x; i < wt.n_scenes; i += blockDim.x) scenes[i] = wt.scenes[i];
   __syncthreads();
   __shared__ float world[kTraceWarps][kWorldFloats];
-    __shared__ uint2 entries[kSharedEntries][kTraceThreads];
+  __shared__ uint2 entries[kSharedEntries][kTraceThreads];
   const uint32_t st = trace_refill<true, false>(
       sq.fetch + bounce, n,
       [&](uint32_t r, V3& o, V3& d, uint32_t& sidx) {
@@ -1994,7 +1994,8 @@ __device__ __forceinline__ void put_radiance(const PathBatch& pb, const WaveTabl
 // the longest path and not the sum over the bounces of each bounce's longest ray.  All lanes of a
 // group shade the same vertex; lane 0 writes.  Samples, arithmetic and the order of a path's
 // radiance additions are those of the per-bounce kernels.  Bound by the latency of a path's steps
-// (0.8 us each) and, from ~16K paths on, by instruction issue (54%).
+// (0.8 us each): the schedulers issue in 37% of the cycles in which they have warps at 3,072 paths, in 42% at
+// 19,200.
 // With kWaveDirect (one sample per pixel, reference or NEE estimator) a path adds its radiance to its
 // pixel itself (accumulate_sample) and the wave needs no other launch.
 enum EstimatorKind : int { kEstPlain, kEstNee, kEstCache };
